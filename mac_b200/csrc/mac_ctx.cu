@@ -200,8 +200,8 @@ static void free_all(Ctx* c) {
   if (c->ev_topo) cudaEventDestroy(c->ev_topo);
   if (c->ev_bins) cudaEventDestroy(c->ev_bins);
   if (c->side) cudaStreamDestroy(c->side);
-  cudaFree(c->csc_off); cudaFree(c->csc_ind); cudaFree(c->csc_val); cudaFree(c->csc_vec);
-  cudaFree(c->csr_off); cudaFree(c->csr_ind); cudaFree(c->csr_val); cudaFree(c->eb_work);
+  csc_release(c, 0);
+  cudaFree(c->eb_work);
   if (c->stream) cudaStreamDestroy(c->stream);
 }
 

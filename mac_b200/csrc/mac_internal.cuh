@@ -233,10 +233,13 @@ struct Ctx {
   bool system_ready = false;
   // drop-in CSC solver
   int csc_n = 0;
+  char* csc_buf = nullptr;     // the solver's device memory; the arrays below lie in it
+  size_t csc_bytes = 0;
+  int csc_longest = 0;         // entries of the longest column
   int* csc_off = nullptr;
   int* csc_ind = nullptr;
   double* csc_val = nullptr;
-  double* csc_vec = nullptr;   // [7][n] + scalars (CG), [11][n] + scalars (BiCGStab)
+  double* csc_vec = nullptr;   // [7][n] + slots and scalars (CG), [11][n] + scalars (BiCGStab)
   int csc_general = 0;         // 1: not the symmetric negative-diagonal form, solved by BiCGStab
   int* csr_off = nullptr;      // row-major copy for BiCGStab
   int* csr_ind = nullptr;
@@ -598,5 +601,14 @@ int mg_setup(Ctx* c);
 void mg_vcycle(Ctx* c, int update, int part);
 void cg_finish_update(Ctx* c);
 int mg_configure(Ctx* c);
+// Drops the CSC solver's matrix; its device memory too when it is over `keep` bytes.
+void csc_release(Ctx* c, size_t keep);
+// The CSC solve as one resident kernel (mac_csc.cu): rows of at most kCscRow
+// entries; doubles of work space beyond the 2 n of z.
+constexpr int kCscRow = 7;
+constexpr size_t kCscWork = 2 * 16 * 512;
+int csc_cg_resident(cudaStream_t st, int n, const int* off, const int* ind, const double* val, const double* b,
+                    double* x, double* work, const double* flags, double rtol, int max_iters, double* res,
+                    int* enqueued);
 
 }  // namespace mac

@@ -9,8 +9,9 @@
 // in device memory when the first call on a device (or the set-up call with
 // n = 0) looks up its address, so that call needs 2.5 MiB of free device
 // memory, and no later call needs any. It runs the CG kernels of
-// mac_csc_solve (k_csc_diag, k_csc_vec, k_csc_spmv) in the same order, after
-// a check that the matrix has the symmetric negative-diagonal form CG needs.
+// mac_csc_solve in the same order (the resident solve of mac_csc.cu; for rows
+// longer than its kCscRow k_csc_diag, k_csc_vec, k_csc_spmv), after a check
+// that the matrix has the symmetric negative-diagonal form CG needs.
 #include <cmath>
 #include <mutex>
 
@@ -26,9 +27,13 @@ __global__ void k_csc_diag(int n, const int* __restrict__ off, const int* __rest
                            const double* __restrict__ val, double* dinv);
 __global__ void k_csc_vec(int n, int mode, const double* b, double* x, double* r, double* z, double* p,
                           const double* q, const double* dinv, double* scal, double a);
+// Defined with the resident solve (mac_csc.cu).
+__global__ void k_csc_check(int n, const int* __restrict__ off, const int* __restrict__ ind,
+                            const double* __restrict__ val, double* flags);
 
 // Scratch: the work vectors r, z, p, q, dinv (MAC_NOALLOC_MAX_N doubles each,
-// 2.5 MiB in all) followed by 8 reduction slots. Every vector entry a solve
+// 2.5 MiB in all; the resident solve uses z and its exchange slots) followed by
+// 8 reduction slots. Every vector entry a solve
 // reads is written earlier in that solve, so the vectors need no initial
 // value; the reduction slots must be zero when each reduction kernel starts,
 // and the solve clears them itself before every reduction.
@@ -56,39 +61,6 @@ static int scratch_address(double** out) {
   return MAC_OK;
 }
 
-// Flags (slot 7 = 1) a matrix that is not the symmetric negative-diagonal form
-// CG needs: a row index outside [0, n), a diagonal entry that is not negative
-// or not present exactly once, or an off-diagonal (i, j) whose mirror (j, i)
-// is missing or differs. Column i is scanned linearly for the mirror (the
-// reference's columns hold at most 7 entries).
-__global__ void k_csc_check(int n, const int* __restrict__ off, const int* __restrict__ ind,
-                            const double* __restrict__ val, double* scal) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-    const int k0 = off[j], k1 = off[j + 1];
-    bool bad = j == 0 && k0 != 0;
-    int ndiag = 0;
-    if (k1 < k0) bad = true;
-    for (int k = k0; k < k1 && !bad; ++k) {
-      const int i = ind[k];
-      if (i < 0 || i >= n) {
-        bad = true;
-      } else if (i == j) {
-        ndiag += 1;
-        if (!(val[k] < 0)) bad = true;
-      } else {
-        bool found = false;
-        for (int m = off[i]; m < off[i + 1]; ++m)
-          if (ind[m] == j) {
-            found = val[m] == val[k];
-            break;
-          }
-        if (!found) bad = true;
-      }
-    }
-    if (bad || ndiag != 1) scal[7] = 1.0;
-  }
-}
-
 static int read_slots(double* hs, const double* scal, cudaStream_t st) {
   int rc = check(cudaMemcpyAsync(hs, scal, 64, cudaMemcpyDeviceToHost, st));
   return rc ? rc : check(cudaStreamSynchronize(st));
@@ -107,8 +79,19 @@ static int csc_solve_noalloc(cudaStream_t st, int n, const int* off, const int* 
   double hs[8];
   if ((rc = check(cudaMemsetAsync(scal, 0, 64, st)))) return rc;
   k_csc_check<<<g, 256, 0, st>>>(n, off, ind, val, scal);
+  // the resident solve runs right behind the check and returns at once when
+  // the check refused the matrix or found a longer row: one host read in all
+  int enqueued = 0;
+  static_assert(kNoAllocSlots >= 2 * (size_t)MAC_NOALLOC_MAX_N + kCscWork, "z and the exchange slots fit the scratch");
+  if ((rc = csc_cg_resident(st, n, off, ind, val, b, x, v, scal, rtol, max_iters, scal + 4, &enqueued))) return rc;
   if ((rc = check(cudaGetLastError())) || (rc = read_slots(hs, scal, st))) return rc;
-  if (hs[7] != 0.0) return MAC_ERR_MATRIX;
+  if (hs[0] != 0.0) return MAC_ERR_MATRIX;
+  if (enqueued && hs[1] == 0.0) {
+    if (hs[7] != 0.0) return MAC_ERR_TIMEOUT;
+    if (iterations) *iterations = (int)hs[4];
+    if (relres) *relres = hs[6] > 0 ? std::sqrt(hs[5] / hs[6]) : 0.0;
+    return (hs[6] > 0 && !(hs[5] <= rtol * rtol * hs[6])) ? MAC_ERR_NOT_CONVERGED : MAC_OK;
+  }
   k_csc_diag<<<g, 256, 0, st>>>(n, off, ind, val, dinv);
   if ((rc = check(cudaMemsetAsync(scal, 0, 64, st)))) return rc;
   k_csc_vec<<<g, 256, 0, st>>>(n, 0, b, x, r, z, p, q, dinv, scal, 0);

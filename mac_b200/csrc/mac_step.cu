@@ -197,6 +197,30 @@ static int csc_solve_cg(Ctx* c, const double* hb, double* hx) {
   int n = c->csc_n;
   cudaStream_t st = c->stream;
   double* v = c->csc_vec;
+  if (c->csc_longest <= kCscRow) {
+    // the whole solve in one resident kernel: z and its slots, b, x, result
+    const size_t nz = 2 * (size_t)n + kCscWork;
+    double *b = v + nz, *x = b + n, *res = x + n, h[4];
+    int rc = check(cudaMemcpyAsync(b, hb, 8 * (size_t)n, cudaMemcpyHostToDevice, st)), enqueued = 0;
+    if (!rc)
+      rc = csc_cg_resident(st, n, c->csc_off, c->csc_ind, c->csc_val, b, x, v, nullptr, c->prm.rtol, c->prm.max_iters,
+                           res, &enqueued);
+    if (rc) return rc;
+    if (enqueued) {
+      MAC_COUNT(c);
+      rc = check(cudaMemcpyAsync(hx, x, 8 * (size_t)n, cudaMemcpyDeviceToHost, st));
+      if (!rc) rc = check(cudaMemcpyAsync(h, res, 32, cudaMemcpyDeviceToHost, st));
+      if (!rc) rc = check(cudaStreamSynchronize(st));
+      if (rc) return rc;
+      if (h[3] != 0.0) return MAC_ERR_TIMEOUT;
+      c->stats.iterations = (int)h[0];
+      c->stats.total_iterations += (int)h[0];
+      c->stats.solves += 1;
+      c->stats.relres = h[2] > 0 ? std::sqrt(h[1] / h[2]) : 0.0;
+      c->stats.unknowns = n;
+      return (h[2] > 0 && !(h[1] <= c->prm.rtol * c->prm.rtol * h[2])) ? MAC_ERR_NOT_CONVERGED : MAC_OK;
+    }
+  }
   double *b = v, *x = v + n, *r = v + 2 * (size_t)n, *z = v + 3 * (size_t)n, *p = v + 4 * (size_t)n,
          *q = v + 5 * (size_t)n, *dinv = v + 6 * (size_t)n, *scal = v + 7 * (size_t)n;
   int g = grid_for(n, 256);
@@ -454,6 +478,102 @@ static void csc_to_csr(int n, const int* off, const int* ind, const double* val,
     }
 }
 
+// The solver's device memory is one buffer of the context, kept from one
+// factorisation to the next up to kCscKeep bytes (a projection factorises,
+// solves and cleans once a step, and each cudaMalloc and cudaFree waits for
+// the device); a larger one is given back by mac_csc_clean.
+constexpr size_t kCscKeep = (size_t)64 << 20;
+
+void csc_release(Ctx* c, size_t keep) {
+  if (c->csc_bytes > keep) {
+    cudaFree(c->csc_buf);
+    c->csc_buf = nullptr;
+    c->csc_bytes = 0;
+  }
+  c->csc_off = c->csc_ind = c->csr_off = c->csr_ind = nullptr;
+  c->csc_val = c->csc_vec = c->csr_val = nullptr;
+  c->csc_general = 0;
+  c->csc_n = 0;
+}
+
+// Carves the buffer into offsets, indices, values and nvec doubles of vectors.
+static int csc_reserve(Ctx* c, int n, int nnz, size_t nvec, int** off, int** ind, double** val) {
+  auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+  const size_t bo = up(4 * (size_t)(n + 1)), bi = up(4 * (size_t)(nnz ? nnz : 1)), bv = up(8 * (size_t)(nnz ? nnz : 1));
+  const size_t need = bo + bi + bv + 8 * nvec;
+  if (need > c->csc_bytes) {
+    cudaFree(c->csc_buf);
+    c->csc_buf = nullptr;
+    c->csc_bytes = 0;
+    int rc = check(cudaMalloc((void**)&c->csc_buf, need));
+    if (rc) return rc;
+    c->csc_bytes = need;
+  }
+  *off = (int*)c->csc_buf;
+  *ind = (int*)(c->csc_buf + bo);
+  *val = (double*)(c->csc_buf + bo + bi);
+  c->csc_vec = (double*)(c->csc_buf + bo + bi + bv);
+  return MAC_OK;
+}
+
+__global__ void k_csc_check(int n, const int* __restrict__ off, const int* __restrict__ ind,
+                            const double* __restrict__ val, double* flags);
+
+// Columns of at most this many entries are checked on the device, one thread a
+// column (its cost grows with the square of the length).
+constexpr int kCscCheckMax = 64;
+
+static int csc_factorize(Ctx* c, int n, const int* offset, const int* indice, const double* value) {
+  const int nnz = offset[n];
+  int longest = 0;
+  for (int j = 0; j < n; ++j) longest = std::max(longest, offset[j + 1] - offset[j]);
+  cudaStream_t st = c->stream;
+  // vectors of the resident solve (z, its slots, b, x) or of the launch-by-launch one (7)
+  int rc = csc_reserve(c, n, nnz, 7 * (size_t)n + kCscWork + 16, &c->csc_off, &c->csc_ind, &c->csc_val);
+  if (!rc) rc = check(cudaMemcpyAsync(c->csc_off, offset, 4 * (size_t)(n + 1), cudaMemcpyHostToDevice, st));
+  if (!rc) rc = check(cudaMemcpyAsync(c->csc_ind, indice, 4 * (size_t)nnz, cudaMemcpyHostToDevice, st));
+  if (!rc) rc = check(cudaMemcpyAsync(c->csc_val, value, 8 * (size_t)nnz, cudaMemcpyHostToDevice, st));
+  if (rc) return rc;
+  // The reference's pressure matrix (symmetric, negative diagonal) goes to
+  // Jacobi-CG; any other matrix Policy_Solve_Linear_Umfpack would factorise
+  // goes to Jacobi-BiCGStab on a row-major copy. The device compares entry by
+  // entry; a column that repeats a row, and long columns, are left to the host.
+  bool general = false, decided = false;
+  if (longest <= kCscCheckMax) {
+    double f[4];
+    rc = check(cudaMemsetAsync(c->csc_vec, 0, 32, st));
+    if (rc) return rc;
+    k_csc_check<<<std::min(grid_for(n, 256), 1184), 256, 0, st>>>(n, c->csc_off, c->csc_ind, c->csc_val,
+                                                                  c->csc_vec); MAC_COUNT(c);
+    rc = check(cudaGetLastError());
+    if (!rc) rc = check(cudaMemcpyAsync(f, c->csc_vec, 32, cudaMemcpyDeviceToHost, st));
+    if (!rc) rc = check(cudaStreamSynchronize(st));
+    if (rc) return rc;
+    decided = f[2] == 0.0;
+    general = f[0] != 0.0;
+  }
+  if (!decided) general = !csc_symmetric_negdiag(n, offset, indice, value);
+  if (general) {
+    std::vector<int> roff, rind;
+    std::vector<double> rval;
+    csc_to_csr(n, offset, indice, value, roff, rind, rval);
+    rc = csc_reserve(c, n, nnz, 11 * (size_t)n + 8, &c->csr_off, &c->csr_ind, &c->csr_val);
+    if (!rc) rc = check(cudaMemcpyAsync(c->csr_off, roff.data(), 4 * (size_t)(n + 1), cudaMemcpyHostToDevice, st));
+    if (!rc) rc = check(cudaMemcpyAsync(c->csr_ind, rind.data(), 4 * (size_t)nnz, cudaMemcpyHostToDevice, st));
+    if (!rc) rc = check(cudaMemcpyAsync(c->csr_val, rval.data(), 8 * (size_t)nnz, cudaMemcpyHostToDevice, st));
+    if (!rc) rc = check(cudaStreamSynchronize(st));
+    if (rc) return rc;
+  }
+  if (!decided && !general) {
+    // the copies above read the caller's arrays
+    if ((rc = check(cudaStreamSynchronize(st)))) return rc;
+  }
+  c->csc_n = n;
+  c->csc_longest = longest;
+  c->csc_general = general ? 1 : 0;
+  return MAC_OK;
+}
+
 }  // namespace mac
 
 using mac::Ctx;
@@ -624,38 +744,9 @@ int mac_csc_factorize(void* ctx, int n, const int* offset, const int* indice, co
   mac_csc_clean(ctx);
   if (n == 0) return MAC_OK;
   if (!mac::csc_valid(n, offset, indice)) return MAC_ERR_INVALID;
-  int nnz = offset[n];
-  // The reference's pressure matrix (symmetric, negative diagonal) goes to
-  // Jacobi-CG; any other matrix Policy_Solve_Linear_Umfpack would factorise
-  // goes to Jacobi-BiCGStab on a row-major copy.
-  const bool general = !mac::csc_symmetric_negdiag(n, offset, indice, value);
-  const size_t nvec = general ? 11 : 7;
-  int rc = mac::check(cudaMalloc((void**)&c->csc_off, 4 * (size_t)(n + 1)));
-  if (!rc) rc = mac::check(cudaMalloc((void**)&c->csc_ind, 4 * (size_t)(nnz ? nnz : 1)));
-  if (!rc) rc = mac::check(cudaMalloc((void**)&c->csc_val, 8 * (size_t)(nnz ? nnz : 1)));
-  if (!rc) rc = mac::check(cudaMalloc((void**)&c->csc_vec, 8 * (size_t)(nvec * (size_t)n + 8)));
-  if (!rc) rc = mac::check(cudaMemcpyAsync(c->csc_off, offset, 4 * (size_t)(n + 1), cudaMemcpyHostToDevice, c->stream));
-  if (!rc) rc = mac::check(cudaMemcpyAsync(c->csc_ind, indice, 4 * (size_t)nnz, cudaMemcpyHostToDevice, c->stream));
-  if (!rc) rc = mac::check(cudaMemcpyAsync(c->csc_val, value, 8 * (size_t)nnz, cudaMemcpyHostToDevice, c->stream));
-  std::vector<int> roff, rind;
-  std::vector<double> rval;
-  if (general && !rc) {
-    mac::csc_to_csr(n, offset, indice, value, roff, rind, rval);
-    rc = mac::check(cudaMalloc((void**)&c->csr_off, 4 * (size_t)(n + 1)));
-    if (!rc) rc = mac::check(cudaMalloc((void**)&c->csr_ind, 4 * (size_t)(nnz ? nnz : 1)));
-    if (!rc) rc = mac::check(cudaMalloc((void**)&c->csr_val, 8 * (size_t)(nnz ? nnz : 1)));
-    if (!rc) rc = mac::check(cudaMemcpyAsync(c->csr_off, roff.data(), 4 * (size_t)(n + 1), cudaMemcpyHostToDevice, c->stream));
-    if (!rc) rc = mac::check(cudaMemcpyAsync(c->csr_ind, rind.data(), 4 * (size_t)nnz, cudaMemcpyHostToDevice, c->stream));
-    if (!rc) rc = mac::check(cudaMemcpyAsync(c->csr_val, rval.data(), 8 * (size_t)nnz, cudaMemcpyHostToDevice, c->stream));
-  }
-  if (!rc) rc = mac::check(cudaStreamSynchronize(c->stream));
-  if (rc) {
-    mac_csc_clean(ctx);
-    return rc;
-  }
-  c->csc_n = n;
-  c->csc_general = general ? 1 : 0;
-  return MAC_OK;
+  int rc = mac::csc_factorize(c, n, offset, indice, value);
+  if (rc) mac_csc_clean(ctx);
+  return rc;
 }
 
 int mac_csc_solve(void* ctx, int n, const double* b, double* x) {
@@ -666,22 +757,7 @@ int mac_csc_solve(void* ctx, int n, const double* b, double* x) {
 
 int mac_csc_clean(void* ctx) {
   CTX_OR_FAIL();
-  cudaFree(c->csc_off);
-  cudaFree(c->csc_ind);
-  cudaFree(c->csc_val);
-  cudaFree(c->csc_vec);
-  cudaFree(c->csr_off);
-  cudaFree(c->csr_ind);
-  cudaFree(c->csr_val);
-  c->csr_off = nullptr;
-  c->csr_ind = nullptr;
-  c->csr_val = nullptr;
-  c->csc_general = 0;
-  c->csc_off = nullptr;
-  c->csc_ind = nullptr;
-  c->csc_val = nullptr;
-  c->csc_vec = nullptr;
-  c->csc_n = 0;
+  mac::csc_release(c, mac::kCscKeep);
   return MAC_OK;
 }
 
