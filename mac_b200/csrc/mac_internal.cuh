@@ -199,6 +199,11 @@ struct Ctx {
   double mg_scale = 0.6;      // coarse-operator scale of the Galerkin products
   int mg_sweeps0 = 2;         // Jacobi sweeps before and after the coarse correction at level 0 (1 or 2)
   int mg_bulk = 0;            // 1: the V-cycle's first kernel prefetches bricks with cp.async.bulk
+  unsigned long long* res_slots = nullptr;  // the resident solve's arrival count, its value after the last
+                              // solve, and the blocks' parts of a sum
+  int res_grid = 0;           // blocks of the resident solve (0: not available)
+  int res_smem = 0;           // its largest dynamic shared memory
+  int res_cluster = 0;        // one cluster of 16 of its blocks fits
   int bulk_grid = 0;          // its grid (blocks resident on all SMs at once)
   int npart_head = 0;         // partial sums the V-cycle's first kernel left (its grid)
   // learned preconditioner (flexible CG): the network and the previous z
@@ -391,8 +396,8 @@ __device__ inline void load_face_bases(const int* __restrict__ nbr, int b, int64
 }
 
 // A domain brick's row of the brick rows built with the solve's domain list:
-// its pool index and its -x, +x, -y, +y, -z, +z face neighbours (-1 absent),
-// 8 ints. One load round gives a block its brick and face bases (threads 0..5
+// its pool index, its -x, +x, -y, +y, -z, +z face neighbours (-1 absent) and
+// its cell of the dense level 3, 8 ints. One load round gives a block its brick and face bases (threads 0..5
 // stage them, in load_face_bases' order), where the list and the neighbour
 // table take two.
 __device__ inline int load_drow(const int* __restrict__ drow, int64_t* sb) {
@@ -601,6 +606,9 @@ int mg_setup(Ctx* c);
 void mg_vcycle(Ctx* c, int update, int part);
 void cg_finish_update(Ctx* c);
 int mg_configure(Ctx* c);
+int cg_resident(Ctx* c, int* enqueued);
+constexpr int kResMaxBlocks = 160;
+constexpr int kResSlots = 32 + 2 * kResMaxBlocks;
 // Drops the CSC solver's matrix; its device memory too when it is over `keep` bytes.
 void csc_release(Ctx* c, size_t keep);
 // The CSC solve as one resident kernel (mac_csc.cu): rows of at most kCscRow

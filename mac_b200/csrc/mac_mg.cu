@@ -17,6 +17,7 @@
 // preconditioned residual z the CG iteration exchanges stay double.
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <utility>
 
 #include "mac_internal.cuh"
@@ -1710,6 +1711,8 @@ void mg_vcycle(Ctx* c, int update, int part) {
   else mg_vcycle_t<double>(c, update, part);
 }
 
+#include "mac_mg_resident.cuh"
+
 int mg_configure(Ctx* c) {
   int dev = c->prm.device, optin = 0;
   cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
@@ -1733,6 +1736,7 @@ int mg_configure(Ctx* c) {
                                                                       bulk_smem<double>()));
   }
   c->bulk_grid = rc ? 0 : nsm * occ;
+  if (!rc) rc = c->mg_float ? res_configure_t<float>(c, nsm, optin) : res_configure_t<double>(c, nsm, optin);
   return rc;
 }
 

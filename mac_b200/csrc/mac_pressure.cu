@@ -47,6 +47,8 @@ int alloc_solver(Ctx* c) {
   A(dalloc(&c->q, nc));
   A(dalloc(&c->dbl, c->cap_bricks));
   A(dalloc(&c->drow, (size_t)c->cap_bricks * 8));
+  A(dalloc(&c->res_slots, kResSlots));
+  if (rc == MAC_OK) A(check(cudaMemset(c->res_slots, 0, 8 * kResSlots)));
   A(dalloc(&c->coarse_inv, 64 * 64));
   A(dalloc(&c->coarse_ok, 1));
   if (rc == MAC_OK) A(check(cudaMemset(c->coarse_ok, 0, sizeof(int))));
@@ -76,6 +78,7 @@ void free_solver(Ctx* c) {
   cudaFree(c->q); cudaFree(c->pd2); cudaFree(c->partial); cudaFree(c->dbl); cudaFree(c->dense_buf);
   cudaFree(c->dbl_map); cudaFree(c->dbl_cnt); cudaFree(c->drow);
   cudaFree(c->zold);
+  cudaFree(c->res_slots);
   cudaFree(c->coarse_inv);
   cudaFree(c->coarse_ok);
   for (int l = 0; l < kLevels; ++l) {
@@ -256,7 +259,8 @@ __global__ void __launch_bounds__(kOrderBlock) k_order_write(const int* __restri
   if (b >= 0) dbl[off[blockIdx.x] + before + __popc(bal & ((1u << lane) - 1u))] = b;
 }
 
-__global__ void k_drow(const int* __restrict__ dbl, int nd, const int* __restrict__ nbr, int* __restrict__ drow) {
+__global__ void k_drow(const int* __restrict__ dbl, int nd, const int* __restrict__ nbr, const int* __restrict__ bkey,
+                       DenseGrid g, int* __restrict__ drow) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 8 * (int64_t)nd) return;
   const int k = (int)(t & 7);
@@ -267,14 +271,15 @@ __global__ void k_drow(const int* __restrict__ dbl, int nd, const int* __restric
   } else if (k < 7) {
     const int f = k - 1, d = (f & 1) ? 1 : -1, ax = f >> 1;
     v = nbr[(size_t)b * kNbr + nbr_index(ax == 0 ? d : 0, ax == 1 ? d : 0, ax == 2 ? d : 0)];
+  } else {
+    v = (int)g.index(bkey[3 * b], bkey[3 * b + 1], bkey[3 * b + 2]);
   }
   drow[t] = v;
 }
 
-static int order_domain_bricks(Ctx* c) {
+// The domain bricks' bounding box (level 3 of the multigrid has a cell per brick of it).
+static DenseGrid domain_box(const Ctx* c) {
   const int* bb = c->hs->bbox;
-  const int nd = c->ndom_host;
-  if (nd <= 1) return MAC_OK;
   DenseGrid g;
   g.x0 = bb[0];
   g.y0 = bb[1];
@@ -282,6 +287,13 @@ static int order_domain_bricks(Ctx* c) {
   g.nx = bb[3] - bb[0] + 1;
   g.ny = bb[4] - bb[1] + 1;
   g.nz = bb[5] - bb[2] + 1;
+  return g;
+}
+
+static int order_domain_bricks(Ctx* c) {
+  const int nd = c->ndom_host;
+  if (nd <= 1) return MAC_OK;
+  const DenseGrid g = domain_box(c);
   const int64_t n = (int64_t)g.nx * g.ny * g.nz;
   if (g.nx < 1 || g.ny < 1 || g.nz < 1 || n > kOrderMaxSlots) return MAC_OK;
   const int64_t nb = (n + kOrderBlock - 1) / kOrderBlock;
@@ -826,7 +838,8 @@ int setup_system(Ctx* c) {
   c->stats.unknowns = c->hs->nunknown;
   if ((rc = order_domain_bricks(c))) return rc;
   if (c->ndom_host > 0) {
-    k_drow<<<grid_for(8 * (int64_t)c->ndom_host, 256), 256, 0, st>>>(c->dbl, c->ndom_host, c->nbr, c->drow); MAC_COUNT(c);
+    k_drow<<<grid_for(8 * (int64_t)c->ndom_host, 256), 256, 0, st>>>(c->dbl, c->ndom_host, c->nbr, c->bkey,
+                                                                               domain_box(c), c->drow); MAC_COUNT(c);
   }
   if (c->ndom_host > 0 && c->prm.solver != MAC_SOLVER_CG_FP64) {
     rc = mg_setup(c);
@@ -924,6 +937,18 @@ int project_field(Ctx* c, double* const* U, const double* const* D) {
     double rr_prev = -1;  // r.r of the iteration before the last one read back
     while (true) {
       const bool fold = mg && !learned;
+      if (fold && first) {
+        // systems of up to about a thousand bricks: every iteration in one kernel
+        int resident = 0;
+        prof_begin(c, PH_VCYCLE);
+        rc = cg_resident(c, &resident);
+        prof_end(c, PH_VCYCLE);
+        if (rc) return rc;
+        if (resident) {
+          lagged = true;
+          break;
+        }
+      }
       prof_begin(c, PH_VCYCLE);
       if (learned) {
         if ((rc = learned_precondition(c, first))) return rc;
