@@ -111,8 +111,8 @@ __device__ __forceinline__ void fence_barrier_init() {
 
 // ------------------------------------------------------- convolution (M = voxels)
 // MODE 0: forward, out = act(conv(in) + bias), B = W K-major.
-// MODE 1: input gradient, out = conv(g * gate) with negated taps, B = W MN-major;
-//         output channels [0, c1) go to d1 and [c1, NC) to d2.
+// MODE 1: input gradient, out = conv(g) with negated taps, B = W MN-major;
+//         output channels [0, c1) go to d1, gated, and [c1, NC) to d2.
 constexpr int kConvStages = 4;
 
 template <int KC, int NC>
@@ -170,13 +170,7 @@ __global__ void __launch_bounds__(128) k_conv(ConvArgs a) {
 #pragma unroll
     for (int c = 0; c < KC / 8; ++c) {
       uint4 val = make_uint4(0, 0, 0, 0);
-      if (inb) {
-        val = gather8(a.s1, a.s2, c, n, sz, sy, sx, a.d, a.h, a.w);
-        if (MODE == 1 && a.gate) {
-          size_t gv = (((size_t)n * a.d + sz) * a.h + sy) * a.w + sx;
-          val = gate8(val, ldg16(a.gate + gv * KC + c * 8));
-        }
-      }
+      if (inb) val = gather8(a.s1, a.s2, c, n, sz, sy, sx, a.d, a.h, a.w);
       *reinterpret_cast<uint4*>(As + (tid >> 3) * SBO + c * 128 + (tid & 7) * 16) = val;
     }
     // weights of tap t: global rows of CH chunks; forward rows are output
@@ -237,6 +231,10 @@ __global__ void __launch_bounds__(128) k_conv(ConvArgs a) {
         dst = a.d1 + (size_t)v * a.c1 + c0;
       else
         dst = a.d2 + (size_t)v * (NC - a.c1) + (c0 - a.c1);
+      if (MODE == 1 && a.gate && c0 < a.c1) {
+        pk[0] = gate8(pk[0], ldg16(a.gate + (size_t)v * a.c1 + c0));
+        pk[1] = gate8(pk[1], ldg16(a.gate + (size_t)v * a.c1 + c0 + 8));
+      }
       reinterpret_cast<uint4*>(dst)[0] = pk[0];
       reinterpret_cast<uint4*>(dst)[1] = pk[1];
     }
@@ -249,6 +247,7 @@ __global__ void __launch_bounds__(128) k_conv(ConvArgs a) {
 }
 
 // ------------------------------------- forward 3x3x3 convolution, staged tile
+// (64 -> 64 channels, whose weights do not fit beside k_conv_march's planes.)
 // A CTA computes a tile of 8 (x) x 16 (y) x 1 (z) output voxels (M = 128).
 // Its input box with a one-voxel halo, 10 x 18 x 3 voxels x KC channels, is
 // gathered from global memory once (concatenation and nearest upsampling of
@@ -396,7 +395,7 @@ __global__ void __launch_bounds__(128) k_conv_tile(ConvArgs a) {
 }
 
 // ------------------------------------------------ weight gradient (K = voxels)
-// dW[tap][co][ci] += sum_v in[v + off(tap)][ci] * (g * gate)[v][co]; a CTA owns
+// dW[tap][co][ci] += sum_v in[v + off(tap)][ci] * g[v][co]; a CTA owns
 // 16 (tap, 8-channel group) row blocks = 128 GEMM rows and a range of voxels.
 constexpr int kWgStages = 4;
 constexpr int kWgK = 64;  // voxels per stage
@@ -469,10 +468,7 @@ __global__ void __launch_bounds__(128) k_wgrad(WgradArgs a) {
       const int nch = (tid >> 6) + 2 * j;
       if (nch < COUT / 8) {
         uint4 val = make_uint4(0, 0, 0, 0);
-        if (valid) {
-          val = ldg16(a.g + (size_t)v * COUT + nch * 8);
-          if (a.gate) val = gate8(val, ldg16(a.gate + (size_t)v * COUT + nch * 8));
-        }
+        if (valid) val = ldg16(a.g + (size_t)v * COUT + nch * 8);
         *reinterpret_cast<uint4*>(Bs + nch * SBO + row_off) = val;
       }
     }
@@ -516,10 +512,378 @@ __global__ void __launch_bounds__(128) k_wgrad(WgradArgs a) {
   if (warp == 0) umma::tmem_dealloc(tmem, TCOLS);
 }
 
+// --------------------------------- 3x3x3 convolutions marching along z
+// A CTA owns an 8 (x) x 16 (y) tile of voxels and walks it through a run of z
+// planes. The input planes of the tile with a one-voxel halo (10 x 18 voxels x
+// KC channels) pass through a ring of four in shared memory, in the no-swizzle
+// K-major layout [channel group][y][x] x 16 bytes: a tap's A operand is the
+// planes seen from another start address (M-adjacent core matrices 160 bytes
+// apart, K-adjacent ones a channel group). Each plane is gathered once a run
+// where a box per plane gathers three, the next plane's loads are in flight in
+// registers while the tensor core works on this one, the epilogue of the plane
+// before (bias, ReLU, BF16 store) runs meanwhile, and the weights of all taps
+// are staged once a run. Two accumulators alternate in tensor memory. The
+// accumulation visits taps and K steps in k_conv's order.
+//
+// MODE 0 is the forward convolution, MODE 1 the input gradient (negated taps, B
+// MN-major), as in k_conv. What bounds it is the tensor core's
+// reading of A from shared memory: 27 KC/16 operands of 4 KB a plane. Measured
+// on one B200 (before: a box per output plane, or a gather per tap in MODE 1):
+// forward at 128^3, 16 -> 16 channels 166 -> 108 us, 32 -> 16 569 -> 320 us;
+// input gradient of 16 x 64^3, 16 -> 16 812 -> 231 us.
+constexpr int kPlX = 10, kPlY = 18, kPlVox = kPlX * kPlY, kRing = 4;
+
+template <int KC, int NC>
+__host__ __device__ constexpr int march_smem() {
+  return kRing * KC * kPlVox * 2 + 27 * NC * KC * 2 + 128;
+}
+
+template <int KC, int NC, int MODE>
+__global__ void __launch_bounds__(128) k_conv_march(ConvArgs a, int zrun) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  constexpr int G = KC / 8, PLANE = G * kPlVox * 16, CH = (G * kPlVox + 127) / 128;
+  constexpr int NB = CH > 6 ? 6 : CH;  // chunks of a plane held in registers at a time
+  constexpr uint32_t LBO_A = kPlVox * 16, SBO_A = kPlX * 16, SBO_B = (KC / 8) * 128;
+  constexpr uint32_t ACC = NC < 16 ? 16 : NC, TCOLS = 2 * ACC < 32 ? 32 : 2 * ACC;
+  constexpr uint32_t IDESC = umma::idesc_bf16(128, NC, 0, MODE);
+  uint8_t* wbuf = smem + kRing * PLANE;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(wbuf + 27 * NC * KC * 2);
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 2);
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tx = (a.w + 7) / 8, ty = (a.h + 15) / 16;
+  int bid = blockIdx.x;
+  const int x0 = (bid % tx) * 8;
+  bid /= tx;
+  const int y0 = (bid % ty) * 16;
+  bid /= ty;
+  const int nz = (a.d + zrun - 1) / zrun;
+  const int z0 = (bid % nz) * zrun, n = bid / nz, z1 = min(a.d, z0 + zrun);
+  if (tid == 0) {
+    umma::mbar_init(&bars[0], 1);
+    umma::mbar_init(&bars[1], 1);
+    fence_barrier_init();
+  }
+  if (warp == 0) umma::tmem_alloc(tslot, TCOLS);
+  // chunk i = tid + 128 q of a plane: channel group i / 180, voxel i % 180
+  auto fetch = [&](int z, int q) -> uint4 {
+    const int i = tid + 128 * q, g = i / kPlVox, vox = i - g * kPlVox, by = vox / kPlX;
+    const int x = x0 - 1 + vox - by * kPlX, y = y0 - 1 + by;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (i < G * kPlVox && z >= 0 && z < a.d && y >= 0 && y < a.h && x >= 0 && x < a.w)
+      v = gather8(a.s1, a.s2, g, n, z, y, x, a.d, a.h, a.w);
+    return v;
+  };
+  auto put = [&](int z, int q, uint4 v) {
+    const int i = tid + 128 * q;
+    if (i < G * kPlVox) *reinterpret_cast<uint4*>(smem + ((z + kRing) % kRing) * PLANE + i * 16) = v;
+  };
+  for (int z = z0 - 1; z <= z0 + 1; ++z)
+#pragma unroll
+    for (int q0 = 0; q0 < CH; q0 += NB) {
+      uint4 v[NB];
+#pragma unroll
+      for (int q = 0; q < NB; ++q) v[q] = q0 + q < CH ? fetch(z, q0 + q) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int q = 0; q < NB; ++q)
+        if (q0 + q < CH) put(z, q0 + q, v[q]);
+    }
+  // weights of all taps: forward rows are output channels (K-major), input-gradient rows are K (MN-major)
+  constexpr int ROWS = MODE ? KC : NC, WCH = MODE ? NC / 8 : KC / 8;
+  for (int i = tid; i < 27 * ROWS * WCH; i += 128) {
+    const int t = i / (ROWS * WCH), rem = i - t * ROWS * WCH, row = rem / WCH, c = rem % WCH;
+    const uint4 v = ldg16(a.wt + (size_t)t * NC * KC + (size_t)row * WCH * 8 + c * 8);
+    const uint32_t off = MODE ? (c * SBO_B + (row >> 3) * 128 + (row & 7) * 16)
+                              : ((row >> 3) * SBO_B + c * 128 + (row & 7) * 16);
+    *reinterpret_cast<uint4*>(wbuf + (size_t)t * NC * KC * 2 + off) = v;
+  }
+  umma::fence_before_sync();
+  __syncthreads();
+  umma::fence_after_sync();
+  const uint32_t tmem = *tslot;
+  const int mx = x0 + (tid & 7), my = y0 + (tid >> 3);  // TMEM lane = tile row: x = lane & 7, y = lane >> 3
+  const bool valid = mx < a.w && my < a.h;
+  auto epilogue = [&](int z) {
+    const size_t v = (((size_t)n * a.d + z) * a.h + my) * a.w + mx;
+    const uint32_t trow = tmem + ((z - z0) & 1) * ACC + ((uint32_t)(warp * 32) << 16);
+#pragma unroll
+    for (int c0 = 0; c0 < NC; c0 += 16) {
+      float f[16];
+      umma::tmem_ld16(trow + c0, f);
+      if (!valid) continue;
+      if (MODE == 0) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          if (a.bias) f[i] += a.bias[c0 + i];
+          if (a.relu) f[i] = fmaxf(f[i], 0.0f);
+        }
+      }
+      uint4 pk[2];
+      uint32_t* w32 = reinterpret_cast<uint32_t*>(pk);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        __nv_bfloat162 b2 = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+        w32[i] = *reinterpret_cast<uint32_t*>(&b2);
+      }
+      bf16* dst = c0 < a.c1 ? a.d1 + v * a.c1 + c0 : a.d2 + v * (NC - a.c1) + (c0 - a.c1);
+      if (MODE == 1 && a.gate && c0 < a.c1) {
+        pk[0] = gate8(pk[0], ldg16(a.gate + v * a.c1 + c0));
+        pk[1] = gate8(pk[1], ldg16(a.gate + v * a.c1 + c0 + 8));
+      }
+      reinterpret_cast<uint4*>(dst)[0] = pk[0];
+      reinterpret_cast<uint4*>(dst)[1] = pk[1];
+    }
+  };
+  bool ok = true;
+  for (int z = z0; z < z1; ++z) {
+    umma::fence_before_sync();  // the epilogue's reads of the accumulator this plane overwrites
+    umma::fence_async_smem();
+    ok = __syncthreads_and(ok);
+    if (!ok) break;
+    const int k = z - z0;
+    if (tid == 0) {
+      umma::fence_after_sync();
+      const uint32_t b0 = umma::smem_addr(wbuf), acc = tmem + (k & 1) * ACC;
+      for (int t = 0; t < 27; ++t) {
+        int dz, dy, dx;
+        tap_offset(t, 27, dz, dy, dx);
+        if (MODE == 1) {
+          dz = -dz;
+          dy = -dy;
+          dx = -dx;
+        }
+        const uint32_t at = umma::smem_addr(smem) + ((z + dz + kRing) % kRing) * PLANE + ((1 + dy) * kPlX + 1 + dx) * 16;
+        const uint32_t bt = b0 + t * NC * KC * 2;
+#pragma unroll
+        for (int ks = 0; ks < KC / 16; ++ks)
+          umma::mma(acc, umma::desc(at + ks * 2 * LBO_A, LBO_A, SBO_A), umma::desc(bt + ks * 256, 128, SBO_B), IDESC,
+                    (t > 0 || ks > 0) ? 1u : 0u);
+      }
+      umma::commit(&bars[k & 1]);
+    }
+    // plane z + 2 replaces plane z - 2, which the MMAs of plane z - 1 were the last to read
+    const bool more = z + 1 < z1;
+    uint4 v[NB];
+    if (more) {
+#pragma unroll
+      for (int q = 0; q < NB; ++q) v[q] = fetch(z + 2, q);
+    }
+    if (k > 0) {
+      ok = umma::mbar_wait(&bars[(k - 1) & 1], ((k - 1) >> 1) & 1);
+      umma::fence_after_sync();
+    }
+    if (more) {
+#pragma unroll
+      for (int q = 0; q < NB; ++q) put(z + 2, q, v[q]);
+#pragma unroll
+      for (int q0 = NB; q0 < CH; q0 += NB) {
+#pragma unroll
+        for (int q = 0; q < NB; ++q) v[q] = q0 + q < CH ? fetch(z + 2, q0 + q) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int q = 0; q < NB; ++q)
+          if (q0 + q < CH) put(z + 2, q0 + q, v[q]);
+      }
+    }
+    if (k > 0 && __all_sync(0xffffffffu, ok)) epilogue(z - 1);
+  }
+  const int last = z1 - 1 - z0;
+  if (ok) ok = umma::mbar_wait(&bars[last & 1], (last >> 1) & 1);
+  umma::fence_after_sync();
+  if (__syncthreads_and(ok)) epilogue(z1 - 1);
+  else if (tid == 0) atomicExch(a.err, 1);
+  umma::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) umma::tmem_dealloc(tmem, TCOLS);
+}
+
+// --------------------------------------- 3x3x3 weight gradient from staged lines
+// dW[tap][co][ci] += sum_v in[v + off(tap)][ci] * g[v][co]. A CTA takes
+// one group of eight input channels and a range of voxels v in linear order (the
+// ranges k_wgrad takes) and walks the input lines they touch, L whole x-lines of
+// one plane a step, keeping its products in one tensor-memory accumulator of 128
+// rows x 3 COUT columns until the end. Row blocks j = 3 (dy + 1) + dx + 1 = 0..8
+// are the nine in-plane taps (rows 72.. are not used): a line is staged in three
+// x-shifted copies SBO bytes apart, so that row block j of the A operand
+// (MN-major: eight channels by eight voxels) starts j SBO behind the first one's.
+// The columns are the three dz: the B operand holds g of the planes z + 1, z and
+// z - 1 of the step's lines, so that one MMA of 16 voxels feeds all 27 taps where
+// k_wgrad gathers a row block from global memory for each (an MMA of 128 rows
+// takes about 80 cycles up to 48 columns: A's reading from shared memory bounds
+// it). Lines are padded to a multiple of 16 voxels with zeros, and g is 0 off the
+// range. Every sum adds the same 16-voxel products in the same order as k_wgrad's
+// where w is a multiple of 16 (tensor memory rounds towards zero, so the order
+// and the length of a sum are part of its value: 4e-5 apart with other ranges),
+// with one atomic per weight and CTA at the end. Two stages alternate; one warp
+// issues the MMAs of a step while sixteen load the next. Measured on one B200
+// (before: k_wgrad), 16 x 64^3 samples: the four layers of 16 columns 11.2 -> 2.5
+// ms, of 32 columns (half resolution) 4.2 -> 1.1 ms.
+constexpr int kWlLoad = 512;  // loading threads; a further warp issues the MMAs
+constexpr int kWlIn = 2;      // chunks of input lines a thread carries
+constexpr int kWlVox = 256;   // voxels of a step, padding included
+constexpr int kWlPad = 16;    // bytes between copies: row blocks start in different banks
+constexpr int kWlMaxW = kWlVox / 2;  // widest line: one of COUT = 64 is a whole step
+static_assert(4 * (kWlMaxW + 2) <= kWlLoad * kWlIn, "the lines of the widest step fit the threads' chunks");
+
+template <int COUT>
+__host__ __device__ constexpr int wl_vox() { return COUT == 64 ? kWlVox / 2 : kWlVox; }
+// Bytes of a stage: L + 2 lines (three more that row blocks 9..15 reach past the last), then g of three planes.
+template <int COUT>
+__host__ __device__ inline int wl_stage(int w, int L) {
+  const int w16 = (w + 15) / 16 * 16;
+  return (L + 5) * 3 * (w16 * 16 + kWlPad) + 3 * (COUT / 8) * (L * w16 * 16 + kWlPad);
+}
+
+template <int COUT>
+__global__ void __launch_bounds__(kWlLoad + 32) k_wgrad_lines(WgradArgs a, int cin, int L) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ __align__(8) uint64_t bars[2];
+  __shared__ uint32_t tslot;
+  constexpr int GN = 3 * (COUT / 8) * wl_vox<COUT>() / kWlLoad;  // chunks of g a thread carries
+  constexpr uint32_t TCOLS = 3 * COUT <= 64 ? 64 : (3 * COUT <= 128 ? 128 : 256);
+  constexpr uint32_t IDESC = umma::idesc_bf16(128, 3 * COUT, 1, 1);
+  const int tid = threadIdx.x, warp = tid >> 5, grp = blockIdx.y;
+  const bool loads = tid < kWlLoad;
+  const int w16 = (a.w + 15) / 16 * 16, cs = w16 * 16 + kWlPad, gofs = (L + 5) * 3 * cs;
+  const int gstride = L * w16 * 16 + kWlPad, stage = gofs + 3 * (COUT / 8) * gstride, wx = a.w + 2;
+  if (tid == 0) {
+    umma::mbar_init(&bars[0], 1);
+    umma::mbar_init(&bars[1], 1);
+    fence_barrier_init();
+  }
+  if (warp == 0) umma::tmem_alloc(&tslot, TCOLS);
+  for (int i = tid; i < 2 * stage / 16; i += kWlLoad + 32) reinterpret_cast<uint4*>(smem)[i] = make_uint4(0, 0, 0, 0);
+  umma::fence_before_sync();
+  __syncthreads();
+  umma::fence_after_sync();
+  const uint32_t tmem = tslot;
+  const int V = a.n * a.d * a.h * a.w;
+  const int v0 = blockIdx.x * a.vox_per_cta, v1 = min(V, v0 + a.vox_per_cta);
+  // input lines of the range: its own and a plane before and after
+  const int l0 = max(0, v0 / a.w - a.h), l1 = v0 < v1 ? min(V / a.w, (v1 - 1) / a.w + 1 + a.h) : 0;
+  struct Step {
+    int line, y, z, n, cnt;
+  };
+  // the step that starts at an input line: lines of one plane
+  auto at = [&](int line) -> Step {
+    Step s;
+    s.line = line;
+    const int zn = line / a.h;
+    s.y = line - zn * a.h;
+    s.n = zn / a.d;
+    s.z = zn - s.n * a.d;
+    s.cnt = min(min(L, a.h - s.y), l1 - line);
+    return s;
+  };
+  // this thread's chunks of a step, the same in every step: input line l and
+  // x + 1 (l past the last: none); g's plane dz and channels c as one index b,
+  // line and x (b past the last: none)
+  int il[kWlIn], ibx[kWlIn], gb[GN], gl[GN], gx[GN];
+#pragma unroll
+  for (int q = 0; q < kWlIn; ++q) {
+    const int i = tid + kWlLoad * q;
+    il[q] = i / wx;
+    ibx[q] = i - il[q] * wx;
+  }
+#pragma unroll
+  for (int q = 0; q < GN; ++q) {
+    const int i = tid + kWlLoad * q, k = i % (L * w16);
+    gb[q] = i / (L * w16);
+    gl[q] = k / w16;
+    gx[q] = k - gl[q] * w16;
+  }
+  uint4 vi[kWlIn], vg[GN];
+  auto fetch = [&](const Step& s) {
+#pragma unroll
+    for (int q = 0; q < kWlIn; ++q) {
+      const int x = ibx[q] - 1, y = s.y - 1 + il[q];
+      vi[q] = make_uint4(0, 0, 0, 0);
+      if (il[q] < L + 2 && x >= 0 && x < a.w && y >= 0 && y < a.h)
+        vi[q] = gather8(a.s1, a.s2, grp, s.n, s.z, y, x, a.d, a.h, a.w);
+    }
+#pragma unroll
+    for (int q = 0; q < GN; ++q) {
+      const int dz = gb[q] / (COUT / 8) - 1, c = gb[q] % (COUT / 8), z = s.z - dz;
+      const int v = (s.line - dz * a.h + gl[q]) * a.w + gx[q];
+      const bool in = gb[q] < 3 * (COUT / 8) && z >= 0 && z < a.d && gl[q] < s.cnt && gx[q] < a.w && v >= v0 && v < v1;
+      vg[q] = in ? ldg16(a.g + (size_t)v * COUT + c * 8) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  auto put = [&](uint8_t* st) {
+#pragma unroll
+    for (int q = 0; q < kWlIn; ++q) {
+      if (il[q] >= L + 2) continue;
+      uint8_t* row = st + il[q] * 3 * cs;
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+        if (ibx[q] >= c && ibx[q] - c < a.w) *reinterpret_cast<uint4*>(row + c * cs + (ibx[q] - c) * 16) = vi[q];
+    }
+#pragma unroll
+    for (int q = 0; q < GN; ++q)
+      if (gb[q] < 3 * (COUT / 8))
+        *reinterpret_cast<uint4*>(st + gofs + gb[q] * gstride + (gl[q] * w16 + gx[q]) * 16) = vg[q];
+  };
+  bool ok = true;
+  int cnt = 0;  // steps multiplied so far
+  if (l1 > l0) {
+    Step s = at(l0);
+    if (loads) {
+      fetch(s);
+      put(smem);
+    }
+    while (true) {
+      const int next = s.line + s.cnt, lines = s.cnt;
+      if (next < l1) s = at(next);
+      umma::fence_async_smem();
+      ok = __syncthreads_and(ok);
+      if (!ok) break;
+      if (tid == kWlLoad) {
+        umma::fence_after_sync();
+        const uint32_t base = umma::smem_addr(smem + (cnt & 1) * stage);
+        for (int l = 0; l < lines; ++l)
+          for (int c = 0; c < w16 / 16; ++c)
+            umma::mma(tmem, umma::desc(base + l * 3 * cs + c * 256, 128, cs),
+                      umma::desc(base + gofs + (l * w16 + 16 * c) * 16, 128, gstride), IDESC,
+                      (cnt > 0 || l > 0 || c > 0) ? 1u : 0u);
+        umma::commit(&bars[cnt & 1]);
+      }
+      if (loads && next < l1) {
+        fetch(s);
+        // the other stage is free once the step before is multiplied
+        if (cnt > 0) ok = umma::mbar_wait(&bars[(cnt - 1) & 1], ((cnt - 1) >> 1) & 1);
+        put(smem + ((cnt + 1) & 1) * stage);
+      }
+      ++cnt;
+      if (next >= l1) break;
+    }
+    if (ok && cnt > 0) ok = umma::mbar_wait(&bars[(cnt - 1) & 1], ((cnt - 1) >> 1) & 1);
+  }
+  umma::fence_after_sync();
+  if (__syncthreads_and(ok)) {
+    const int j = tid >> 3;
+    if (cnt > 0 && warp < 3) {  // warps 0..2 hold the nine taps' rows
+      for (int dz = 0; dz < 3; ++dz)
+#pragma unroll
+        for (int c0 = 0; c0 < COUT; c0 += 16) {
+          float f[16];
+          umma::tmem_ld16(tmem + dz * COUT + c0 + ((uint32_t)(warp * 32) << 16), f);
+          if (j < 9) {
+            float* w = a.dw + ((size_t)(dz * 9 + j) * COUT + c0) * cin + grp * 8 + (tid & 7);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) atomicAdd(w + (size_t)i * cin, f[i]);
+          }
+        }
+    }
+  } else if (tid == 0) {
+    atomicExch(a.err, 1);
+  }
+  umma::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) umma::tmem_dealloc(tmem, TCOLS);
+}
+
 // ------------------------------------------------------------ other kernels
-// db[c] += sum_v (g * gate)[v][c], C channels.
+// db[c] += sum_v g[v][c], C channels.
 template <int C>
-__global__ void k_bias_grad(const bf16* __restrict__ g, const bf16* __restrict__ gate, int V, float* db) {
+__global__ void k_bias_grad(const bf16* __restrict__ g, int V, float* db) {
   constexpr int G = C / 8;
   __shared__ float red[256][8];
   const int cg = threadIdx.x % G;
@@ -527,7 +891,6 @@ __global__ void k_bias_grad(const bf16* __restrict__ g, const bf16* __restrict__
   float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   for (int v = blockIdx.x * lanes + threadIdx.x / G; v < V; v += gridDim.x * lanes) {
     uint4 q = ldg16(g + (size_t)v * C + cg * 8);
-    if (gate) q = gate8(q, ldg16(gate + (size_t)v * C + cg * 8));
     const bf16* b = reinterpret_cast<const bf16*>(&q);
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i] += __bfloat162float(b[i]);
@@ -580,9 +943,9 @@ __global__ void k_pool(const bf16* __restrict__ fine, bf16* __restrict__ coarse,
   }
 }
 
-// fine[v] = (accumulate ? fine[v] : 0) + scale * coarse[parent(v)], C channels.
-__global__ void k_unpool(const bf16* __restrict__ coarse, bf16* fine, int n, int d, int h, int w, int C, float scale,
-                         int accumulate) {
+// fine[v] = gate(fine[v] + scale * coarse[parent(v)]), C channels (gate: 0 where the ReLU output was not positive).
+__global__ void k_unpool(const bf16* __restrict__ coarse, bf16* fine, const bf16* __restrict__ gate, int n, int d,
+                         int h, int w, int C, float scale) {
   const int G = C / 8;
   const long total = (long)n * d * h * w * G;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
@@ -597,8 +960,9 @@ __global__ void k_unpool(const bf16* __restrict__ coarse, bf16* fine, int n, int
     const size_t cidx = (((size_t)nn * (d >> 1) + (z >> 1)) * (h >> 1) + (y >> 1)) * (w >> 1) + (x >> 1);
     uint4 q = ldg16(coarse + cidx * C + cg * 8);
     const bf16* b = reinterpret_cast<const bf16*>(&q);
-    bf16* dst = fine + (((size_t)nn * d + z) * h + y) * w * C + (size_t)x * C + cg * 8;
-    uint4 old = accumulate ? *reinterpret_cast<const uint4*>(dst) : make_uint4(0, 0, 0, 0);
+    const size_t at = (((size_t)nn * d + z) * h + y) * w * C + (size_t)x * C + cg * 8;
+    bf16* dst = fine + at;
+    uint4 old = *reinterpret_cast<const uint4*>(dst);
     const bf16* ob = reinterpret_cast<const bf16*>(&old);
     uint4 out;
     uint32_t* o = reinterpret_cast<uint32_t*>(&out);
@@ -609,7 +973,7 @@ __global__ void k_unpool(const bf16* __restrict__ coarse, bf16* fine, int n, int
       __nv_bfloat162 b2 = __floats2bfloat162_rn(f0, f1);
       o[k] = *reinterpret_cast<uint32_t*>(&b2);
     }
-    *reinterpret_cast<uint4*>(dst) = out;
+    *reinterpret_cast<uint4*>(dst) = gate8(out, ldg16(gate + at));
   }
 }
 
@@ -950,15 +1314,38 @@ static void conv_tile_t(const ConvArgs& a, cudaStream_t st) {
   k_conv_tile<KC, NC><<<(unsigned)tiles, 128, smem, st>>>(a);
 }
 
-// Forward 3x3x3 convolutions through the staged-tile kernel.
-static int conv_tile(int kc, int nc, const ConvArgs& a, cudaStream_t st) {
-  if (kc == 16 && nc == 16) conv_tile_t<16, 16>(a, st);
-  else if (kc == 16 && nc == 32) conv_tile_t<16, 32>(a, st);
-  else if (kc == 32 && nc == 32) conv_tile_t<32, 32>(a, st);
-  else if (kc == 32 && nc == 64) conv_tile_t<32, 64>(a, st);
-  else if (kc == 64 && nc == 64) conv_tile_t<64, 64>(a, st);
-  else if (kc == 64 && nc == 32) conv_tile_t<64, 32>(a, st);
-  else if (kc == 32 && nc == 16) conv_tile_t<32, 16>(a, st);
+// Planes a CTA walks: as long a run as still gives the device a few CTAs an SM
+// (a run stages the weights and two extra planes), in runs of equal length.
+static int march_run(const long tiles, int d, int want) {
+  long runs = (want + tiles - 1) / tiles;
+  if (runs < 1) runs = 1;
+  if (runs > (d + 3) / 4) runs = (d + 3) / 4;
+  return (int)((d + runs - 1) / runs);
+}
+
+template <int KC, int NC, int MODE>
+static void conv_march_t(const ConvArgs& a, cudaStream_t st) {
+  constexpr int smem = march_smem<KC, NC>();
+  cudaFuncSetAttribute(k_conv_march<KC, NC, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  const long tiles = (long)a.n * ((a.h + 15) / 16) * ((a.w + 7) / 8);
+  constexpr int occ = 220 * 1024 / (smem + 1024) < 8 ? 220 * 1024 / (smem + 1024) : 8;
+  const int zrun = march_run(tiles, a.d, 148 * occ);
+  k_conv_march<KC, NC, MODE><<<(unsigned)(tiles * ((a.d + zrun - 1) / zrun)), 128, smem, st>>>(a, zrun);
+}
+
+// 3x3x3 convolutions: marching along z where all taps' weights fit beside the
+// ring of planes; 64 x 64 channels (216 KB of weights, the quarter-resolution
+// layers) keep the staged box (forward) and the gather per tap (input gradient).
+template <int MODE>
+static int conv_march(int kc, int nc, const ConvArgs& a, cudaStream_t st) {
+  if (kc == 16 && nc == 16) conv_march_t<16, 16, MODE>(a, st);
+  else if (kc == 16 && nc == 32) conv_march_t<16, 32, MODE>(a, st);
+  else if (kc == 32 && nc == 32) conv_march_t<32, 32, MODE>(a, st);
+  else if (kc == 32 && nc == 64) conv_march_t<32, 64, MODE>(a, st);
+  else if (kc == 64 && nc == 32) conv_march_t<64, 32, MODE>(a, st);
+  else if (kc == 32 && nc == 16) conv_march_t<32, 16, MODE>(a, st);
+  else if (kc == 64 && nc == 64 && MODE == 0) conv_tile_t<64, 64>(a, st);
+  else if (kc == 64 && nc == 64) conv_t<64, 64, MODE>(a, st);
   else return MAC_ERR_INVALID;
   return MAC_OK;
 }
@@ -986,15 +1373,34 @@ static void wgrad_t(const WgradArgs& a, cudaStream_t st) {
   k_wgrad<CIN, COUT><<<dim3(mtiles, ksplit), 128, smem, st>>>(a);
 }
 
+// Voxels a CTA of a weight gradient sums: the split that gives k_wgrad two CTAs an SM.
+static int wgrad_range(int cin, int taps, long V) {
+  const int mtiles = (taps * (cin / 8) + 15) / 16;
+  const long ksplit = std::max<long>(1, std::min<long>((296 + mtiles - 1) / mtiles, (V + 255) / 256));
+  return (int)(((V + ksplit - 1) / ksplit + kWgK - 1) / kWgK * kWgK);
+}
+
+template <int COUT>
+static void wgrad_lines_t(int cin, WgradArgs a, cudaStream_t st) {
+  const long V = (long)a.n * a.d * a.h * a.w;
+  a.vox_per_cta = wgrad_range(cin, 27, V);
+  const int L = wl_vox<COUT>() / ((a.w + 15) / 16 * 16), smem = 2 * wl_stage<COUT>(a.w, L);
+  cudaFuncSetAttribute(k_wgrad_lines<COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  k_wgrad_lines<COUT><<<dim3((unsigned)((V + a.vox_per_cta - 1) / a.vox_per_cta), cin / 8), kWlLoad + 32, smem,
+                        st>>>(a, cin, L);
+}
+
+static int wgrad_lines(int cin, int cout, const WgradArgs& a, cudaStream_t st) {
+  if (cout == 16) wgrad_lines_t<16>(cin, a, st);
+  else if (cout == 32) wgrad_lines_t<32>(cin, a, st);
+  else if (cout == 64) wgrad_lines_t<64>(cin, a, st);
+  else return MAC_ERR_INVALID;
+  return MAC_OK;
+}
+
 static int wgrad(int cin, int cout, WgradArgs a, cudaStream_t st) {
   const long V = (long)a.n * a.d * a.h * a.w;
-  const int mtiles = (a.taps * (cin / 8) + 15) / 16;
-  long ksplit = (296 + mtiles - 1) / mtiles;
-  const long maxsplit = (V + 255) / 256;
-  if (ksplit > maxsplit) ksplit = maxsplit;
-  if (ksplit < 1) ksplit = 1;
-  long per = (V + ksplit - 1) / ksplit;
-  a.vox_per_cta = (int)((per + kWgK - 1) / kWgK * kWgK);
+  a.vox_per_cta = wgrad_range(cin, a.taps, V);
   if (cin == 16 && cout == 16) wgrad_t<16, 16>(a, st);
   else if (cin == 16 && cout == 32) wgrad_t<16, 32>(a, st);
   else if (cin == 32 && cout == 32) wgrad_t<32, 32>(a, st);
@@ -1006,11 +1412,11 @@ static int wgrad(int cin, int cout, WgradArgs a, cudaStream_t st) {
   return MAC_OK;
 }
 
-static void bias_grad(int c, const bf16* g, const bf16* gate, long V, float* db, cudaStream_t st) {
+static void bias_grad(int c, const bf16* g, long V, float* db, cudaStream_t st) {
   const int blocks = (int)std::min<long>(296, (V * (c / 8) + 255) / 256);
-  if (c == 16) k_bias_grad<16><<<blocks, 256, 0, st>>>(g, gate, (int)V, db);
-  else if (c == 32) k_bias_grad<32><<<blocks, 256, 0, st>>>(g, gate, (int)V, db);
-  else k_bias_grad<64><<<blocks, 256, 0, st>>>(g, gate, (int)V, db);
+  if (c == 16) k_bias_grad<16><<<blocks, 256, 0, st>>>(g, (int)V, db);
+  else if (c == 32) k_bias_grad<32><<<blocks, 256, 0, st>>>(g, (int)V, db);
+  else k_bias_grad<64><<<blocks, 256, 0, st>>>(g, (int)V, db);
 }
 
 struct Net {
@@ -1036,7 +1442,7 @@ struct Net {
   double* loss_hist = nullptr;
   int loss_cap = 0;
   long launches = 0;
-  int staged_conv = 1;  // forward 3x3x3 convolutions through k_conv_tile (0: k_conv)
+  int staged_conv = 1;  // 3x3x3 layers from staged planes (0: every tap gathered: k_conv, k_wgrad)
 };
 
 static size_t level_vox(const Net& t, int l) {
@@ -1122,33 +1528,37 @@ static int fwd(Net& t, int l, int lvl, Src s1, Src s2, bf16* dst, float* f32, cu
   a.f32 = f32;
   a.relu = kLayers[l].relu;
   ++t.launches;
-  if (t.staged_conv && a.taps == 27) return conv_tile(kLayers[l].cin, kLayers[l].cout, a, st);
+  if (t.staged_conv && a.taps == 27) return conv_march<0>(kLayers[l].cin, kLayers[l].cout, a, st);
   return conv_mode<0>(kLayers[l].cin, kLayers[l].cout, a, st);
 }
 
-// Input gradient of layer l from the gradient g at its output (gated by the
-// layer's ReLU output y when it has one); channels [0, c1) to d1, the rest to d2.
-static int bwd_in(Net& t, int l, int lvl, const bf16* g, const bf16* y, bf16* d1, int c1, bf16* d2,
+// Gradients are stored gated: a tensor's gradient is zeroed where its ReLU was
+// when it is written, once, so that the passes that read it (input gradient,
+// weight gradient, bias) do not read the activation beside it.
+// Input gradient of layer l from the gated gradient g at its output; channels
+// [0, c1) to d1, gated by y (the activation d1 is the gradient of; null: no
+// gate), the rest to d2.
+static int bwd_in(Net& t, int l, int lvl, const bf16* g, bf16* d1, const bf16* y, int c1, bf16* d2,
                   cudaStream_t st) {
   ConvArgs a = conv_args(t, l, lvl);
   a.s1 = src(g, kLayers[l].cout);
   a.s2 = none();
-  a.gate = kLayers[l].relu ? y : nullptr;
+  a.gate = y;
   a.d1 = d1;
   a.c1 = c1;
   a.d2 = d2;
   ++t.launches;
+  if (t.staged_conv && a.taps == 27) return conv_march<1>(kLayers[l].cout, kLayers[l].cin, a, st);
   return conv_mode<1>(kLayers[l].cout, kLayers[l].cin, a, st);
 }
 
-// Weight and bias gradients of layer l (input concat(s1, s2), output gradient g, output y).
-static int bwd_w(Net& t, int l, int lvl, Src s1, Src s2, const bf16* g, const bf16* y, cudaStream_t st) {
+// Weight and bias gradients of layer l (input concat(s1, s2), gated output gradient g).
+static int bwd_w(Net& t, int l, int lvl, Src s1, Src s2, const bf16* g, cudaStream_t st) {
   WgradArgs a;
   std::memset(&a, 0, sizeof(a));
   a.s1 = s1;
   a.s2 = s2;
   a.g = g;
-  a.gate = kLayers[l].relu ? y : nullptr;
   a.dw = t.g + t.woff[l];
   a.taps = kLayers[l].taps;
   a.n = t.n;
@@ -1157,8 +1567,10 @@ static int bwd_w(Net& t, int l, int lvl, Src s1, Src s2, const bf16* g, const bf
   a.w = t.w >> lvl;
   a.err = t.err;
   t.launches += 2;
-  int rc = wgrad(kLayers[l].cin, kLayers[l].cout, a, st);
-  bias_grad(kLayers[l].cout, g, a.gate, (long)a.n * a.d * a.h * a.w, t.g + t.boff[l], st);
+  // lines wider than a stage holds keep the gather per tap
+  int rc = t.staged_conv && a.taps == 27 && a.w <= kWlMaxW ? wgrad_lines(kLayers[l].cin, kLayers[l].cout, a, st)
+                                                           : wgrad(kLayers[l].cin, kLayers[l].cout, a, st);
+  bias_grad(kLayers[l].cout, g, (long)a.n * a.d * a.h * a.w, t.g + t.boff[l], st);
   return rc;
 }
 
@@ -1168,9 +1580,10 @@ static void pool(Net& t, int lvl, const bf16* fine, bf16* coarse, int c, float s
   ++t.launches;
 }
 
-static void unpool(Net& t, int lvl, const bf16* coarse, bf16* fine, int c, float scale, int acc, cudaStream_t st) {
+static void unpool(Net& t, int lvl, const bf16* coarse, bf16* fine, const bf16* gate, int c, float scale,
+                   cudaStream_t st) {
   const size_t n = level_vox(t, lvl) * (c / 8);
-  k_unpool<<<grid_1d(n), 256, 0, st>>>(coarse, fine, t.n, t.d >> lvl, t.h >> lvl, t.w >> lvl, c, scale, acc);
+  k_unpool<<<grid_1d(n), 256, 0, st>>>(coarse, fine, gate, t.n, t.d >> lvl, t.h >> lvl, t.w >> lvl, c, scale);
   ++t.launches;
 }
 
@@ -1201,35 +1614,35 @@ static int backward(Net& t, cudaStream_t st) {
   bf16** A = t.act;
   bf16** G = t.grad;
   int rc = cuda_ok(cudaMemsetAsync(t.g, 0, t.np * sizeof(float), st));
-  rc |= bwd_w(t, 12, 0, src(A[D1], 16), none(), G[GOUT], nullptr, st);
-  rc |= bwd_in(t, 12, 0, G[GOUT], nullptr, G[D1], 16, nullptr, st);
-  rc |= bwd_w(t, 11, 0, src(A[C1], 16), none(), G[D1], A[D1], st);
-  rc |= bwd_in(t, 11, 0, G[D1], A[D1], G[C1], 16, nullptr, st);
-  rc |= bwd_w(t, 10, 0, src(A[S1], 16), src(A[U1], 16, 1), G[C1], A[C1], st);
-  rc |= bwd_in(t, 10, 0, G[C1], A[C1], G[S1], 16, G[GUP1], st);
+  rc |= bwd_w(t, 12, 0, src(A[D1], 16), none(), G[GOUT], st);
+  rc |= bwd_in(t, 12, 0, G[GOUT], G[D1], A[D1], 16, nullptr, st);
+  rc |= bwd_w(t, 11, 0, src(A[C1], 16), none(), G[D1], st);
+  rc |= bwd_in(t, 11, 0, G[D1], G[C1], A[C1], 16, nullptr, st);
+  rc |= bwd_w(t, 10, 0, src(A[S1], 16), src(A[U1], 16, 1), G[C1], st);
+  rc |= bwd_in(t, 10, 0, G[C1], G[S1], nullptr, 16, G[GUP1], st);  // S1 takes its skip and pool parts, then the gate
   pool(t, 0, G[GUP1], G[U1], 16, 1.0f, st);
-  rc |= bwd_w(t, 9, 1, src(A[D2], 32), none(), G[U1], nullptr, st);
-  rc |= bwd_in(t, 9, 1, G[U1], nullptr, G[D2], 32, nullptr, st);
-  rc |= bwd_w(t, 8, 1, src(A[C2], 32), none(), G[D2], A[D2], st);
-  rc |= bwd_in(t, 8, 1, G[D2], A[D2], G[C2], 32, nullptr, st);
-  rc |= bwd_w(t, 7, 1, src(A[S2], 32), src(A[U2], 32, 1), G[C2], A[C2], st);
-  rc |= bwd_in(t, 7, 1, G[C2], A[C2], G[S2], 32, G[GUP2], st);
+  rc |= bwd_w(t, 9, 1, src(A[D2], 32), none(), G[U1], st);
+  rc |= bwd_in(t, 9, 1, G[U1], G[D2], A[D2], 32, nullptr, st);
+  rc |= bwd_w(t, 8, 1, src(A[C2], 32), none(), G[D2], st);
+  rc |= bwd_in(t, 8, 1, G[D2], G[C2], A[C2], 32, nullptr, st);
+  rc |= bwd_w(t, 7, 1, src(A[S2], 32), src(A[U2], 32, 1), G[C2], st);
+  rc |= bwd_in(t, 7, 1, G[C2], G[S2], nullptr, 32, G[GUP2], st);
   pool(t, 1, G[GUP2], G[U2], 32, 1.0f, st);
-  rc |= bwd_w(t, 6, 2, src(A[B3], 64), none(), G[U2], nullptr, st);
-  rc |= bwd_in(t, 6, 2, G[U2], nullptr, G[B3], 64, nullptr, st);
-  rc |= bwd_w(t, 5, 2, src(A[A3], 64), none(), G[B3], A[B3], st);
-  rc |= bwd_in(t, 5, 2, G[B3], A[B3], G[A3], 64, nullptr, st);
-  rc |= bwd_w(t, 4, 2, src(A[P2], 32), none(), G[A3], A[A3], st);
-  rc |= bwd_in(t, 4, 2, G[A3], A[A3], G[P2], 32, nullptr, st);
-  unpool(t, 1, G[P2], G[S2], 32, 0.125f, 1, st);
-  rc |= bwd_w(t, 3, 1, src(A[A2], 32), none(), G[S2], A[S2], st);
-  rc |= bwd_in(t, 3, 1, G[S2], A[S2], G[A2], 32, nullptr, st);
-  rc |= bwd_w(t, 2, 1, src(A[P1], 16), none(), G[A2], A[A2], st);
-  rc |= bwd_in(t, 2, 1, G[A2], A[A2], G[P1], 16, nullptr, st);
-  unpool(t, 0, G[P1], G[S1], 16, 0.125f, 1, st);
-  rc |= bwd_w(t, 1, 0, src(A[A1], 16), none(), G[S1], A[S1], st);
-  rc |= bwd_in(t, 1, 0, G[S1], A[S1], G[A1], 16, nullptr, st);
-  rc |= bwd_w(t, 0, 0, src(A[IN0], 16), none(), G[A1], A[A1], st);
+  rc |= bwd_w(t, 6, 2, src(A[B3], 64), none(), G[U2], st);
+  rc |= bwd_in(t, 6, 2, G[U2], G[B3], A[B3], 64, nullptr, st);
+  rc |= bwd_w(t, 5, 2, src(A[A3], 64), none(), G[B3], st);
+  rc |= bwd_in(t, 5, 2, G[B3], G[A3], A[A3], 64, nullptr, st);
+  rc |= bwd_w(t, 4, 2, src(A[P2], 32), none(), G[A3], st);
+  rc |= bwd_in(t, 4, 2, G[A3], G[P2], nullptr, 32, nullptr, st);
+  unpool(t, 1, G[P2], G[S2], A[S2], 32, 0.125f, st);
+  rc |= bwd_w(t, 3, 1, src(A[A2], 32), none(), G[S2], st);
+  rc |= bwd_in(t, 3, 1, G[S2], G[A2], A[A2], 32, nullptr, st);
+  rc |= bwd_w(t, 2, 1, src(A[P1], 16), none(), G[A2], st);
+  rc |= bwd_in(t, 2, 1, G[A2], G[P1], nullptr, 16, nullptr, st);
+  unpool(t, 0, G[P1], G[S1], A[S1], 16, 0.125f, st);
+  rc |= bwd_w(t, 1, 0, src(A[A1], 16), none(), G[S1], st);
+  rc |= bwd_in(t, 1, 0, G[S1], G[A1], A[A1], 16, nullptr, st);
+  rc |= bwd_w(t, 0, 0, src(A[IN0], 16), none(), G[A1], st);
   return rc ? MAC_ERR_INVALID : MAC_OK;
 }
 

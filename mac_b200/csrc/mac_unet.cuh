@@ -27,7 +27,7 @@ struct Src {
 
 struct ConvArgs {
   Src s1, s2;                  // K channels = s1.c + s2.c
-  const __nv_bfloat16* gate;   // input gradient: gathered values times (gate > 0)
+  const __nv_bfloat16* gate;   // input gradient: d1 is zeroed where this activation (of d1's tensor) is not positive
   const __nv_bfloat16* wt;     // weights [taps][cout][cin]
   const float* bias;           // forward only
   __nv_bfloat16* d1;           // output channels [0, c1)
@@ -41,8 +41,7 @@ struct ConvArgs {
 
 struct WgradArgs {
   Src s1, s2;                  // the layer's forward input
-  const __nv_bfloat16* g;      // gradient at the layer's output
-  const __nv_bfloat16* gate;   // the layer's output (ReLU) or null
+  const __nv_bfloat16* g;      // gated gradient at the layer's output
   float* dw;                   // [taps][cout][cin], accumulated
   int taps;
   int n, d, h, w;

@@ -56,7 +56,7 @@ class UNet:
                     "mac_unet_set_params")
 
     def set_conv(self, staged=True):
-        """Forward 3x3x3 convolutions through the staged-tile kernel (True) or the per-tap gather."""
+        """3x3x3 layers (forward and backward) from staged planes (True) or with every tap gathered."""
         self._check(self.lib.mac_unet_set_conv(self.h, 1 if staged else 0), "mac_unet_set_conv")
 
     def forward(self, r, mask):
