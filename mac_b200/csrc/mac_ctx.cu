@@ -311,7 +311,7 @@ static int create(const mac_params* p, Ctx** out) {
   A(dalloc(&c->boff, c->cap_bricks + 2));
   A(dalloc(&c->ds, 1));
   if (rc == MAC_OK) A(check(cudaMallocHost((void**)&c->hs, sizeof(Scalars))));
-  if (rc == MAC_OK) A(check(cudaMallocHost((void**)&c->hs_lag, 2 * sizeof(Scalars))));
+  if (rc == MAC_OK) A(check(cudaMallocHost((void**)&c->hs_lag, 3 * sizeof(Scalars))));
   for (int k = 0; k < 2 && rc == MAC_OK; ++k) A(check(cudaEventCreateWithFlags(&c->ev_lag[k], cudaEventDisableTiming)));
   if (rc == MAC_OK) A(alloc_solver(c));
   if (rc == MAC_OK) {

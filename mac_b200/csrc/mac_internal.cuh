@@ -45,6 +45,8 @@ enum ErrBits : int {
 // Field indices of the FP64 per-cell block.
 enum F64 : int { U0X = 0, U0Y, U0Z, U1X, U1Y, U1Z, AX, AY, AZ, PRES, NF64 };
 
+constexpr int kDepthBatch = 6;  // depth relaxation launches between two reads of their marks
+
 struct Scalars {
   int32_t nlive;
   int32_t nlive_new;
@@ -68,7 +70,9 @@ struct Scalars {
   int32_t pad_;
   unsigned long long bad_reads;  // particles whose stencil touched a missing cell
   unsigned long long np_new;     // particle count after the removal pass (depth composition)
-  int32_t dchanged;              // a depth relaxation launch lowered some depth
+  int32_t dchanged[kDepthBatch]; // launch k of a batch of depth relaxations lowered some depth
+  unsigned long long cfl_count;  // fluid cells counted by the time-step pass so far
+  int32_t cfl_blocks;            // its blocks that are done
   int32_t pad2_;
 };
 
@@ -230,7 +234,10 @@ struct Ctx {
   // scalars
   Scalars* ds = nullptr;      // device
   Scalars* hs = nullptr;      // pinned host mirror
-  Scalars* hs_lag = nullptr;  // [2] pinned: the scalars after the last two CG iterations
+  int lag_pending = 0;        // hs_lag[2] holds a projection's scalars that nothing has looked at
+  int lag_status = 0;         // the outcome of that projection, once read
+  Scalars* hs_lag = nullptr;  // [3] pinned: the scalars after the last two CG iterations, and after a projection
+                              // whose outcome is read with the next one's
   cudaEvent_t ev_lag[2] = {};
   int nlive_host = 0;
   int64_t np_host = 0;
@@ -296,19 +303,24 @@ __device__ __forceinline__ void pdl_entry() {
 // launches back wrote; it writes nothing to global memory, and every thread
 // reaches pdl_entry() before it may return.
 
+// On stream st: as a dependent launch on the context's own stream only.
 template <class... P, class... A>
-inline void launch_k(const Ctx* c, void (*k)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
+inline void launch_on(const Ctx* c, cudaStream_t st, void (*k)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
-  cfg.stream = c->stream;
+  cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = c->pdl ? 1 : 0;
+  cfg.numAttrs = c->pdl && st == c->stream ? 1 : 0;
   cudaLaunchKernelEx(&cfg, k, static_cast<A&&>(args)...);
+}
+template <class... P, class... A>
+inline void launch_k(const Ctx* c, void (*k)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
+  launch_on(c, c->stream, k, grid, block, smem, static_cast<A&&>(args)...);
 }
 
 // ---------------------------------------------------------------- helpers
@@ -579,8 +591,11 @@ int rebuild_index(Ctx* c);
 int read_scalars(Ctx* c);
 int forces(Ctx* c, int ib);
 int rk2tvd(Ctx* c);
-int project(Ctx* c, int ib);
-int project_field(Ctx* c, double* const* U, const double* const* D);
+// more = 1: another projection of the same system follows before the caller
+// looks at the outcome (RK2-TVD): no divergence check, and the outcome may be
+// read with the next one's (Ctx::lag_pending).
+int project(Ctx* c, int ib, int more);
+int project_field(Ctx* c, double* const* U, const double* const* D, int more = 0);
 int extrapolate_field(Ctx* c, double* const* F);
 int forces_add(Ctx* c, const double* const* U);
 int rk_all_stage_update(Ctx* c, int stage, const double* const* U);

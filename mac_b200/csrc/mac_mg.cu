@@ -1211,16 +1211,23 @@ __device__ void blk_restrict(const DView<T>& F, const T* fe, const DView<T>& C) 
 // elimination without pivoting (the operator is symmetric positive definite
 // once a cell without a stencil is given a unit row). ok = 0 when a pivot is
 // not positive (no Dirichlet cell anywhere: the V-cycle then keeps Jacobi sweeps).
+// A latency chain of n steps on one SM: thread (i, q) = (tid / 16, tid % 16)
+// keeps the entries (i, q + 16 m) in registers, a step's pivot row (divided by
+// its owners) and column pass through double-buffered shared memory, one barrier
+// a step where the matrix in shared memory took three (64 cells: 86 -> 79 us).
 template <class T>
 __global__ void __launch_bounds__(1024) kd_coarsest_inverse(DView<T> L, double* inv, int* ok) {
+  pdl_entry();
   __shared__ double A[64 * 64];
-  __shared__ double colk[64];
+  __shared__ double row[2][64], col[2][64];
+  __shared__ int bad[2];
   const int n = (int)L.n;
   if (n > 64) {
     if (threadIdx.x == 0) *ok = 0;
     return;
   }
   for (int t = threadIdx.x; t < 64 * 64; t += blockDim.x) A[t] = 0.0;
+  if (threadIdx.x < 2) bad[threadIdx.x] = 0;
   __syncthreads();
   if ((int)threadIdx.x < n) {
     const int i = threadIdx.x;
@@ -1244,28 +1251,39 @@ __global__ void __launch_bounds__(1024) kd_coarsest_inverse(DView<T> L, double* 
       }
     }
   }
+  __syncthreads();
+  const int i = threadIdx.x >> 4, q = threadIdx.x & 15;
+  double v[4];
+#pragma unroll
+  for (int m = 0; m < 4; ++m) v[m] = A[i * 64 + q + 16 * m];
   for (int k = 0; k < n; ++k) {
+    const int b = k & 1, km = k >> 4;
+    // the pivot: entry (k, k), in lane k % 16 of row k's sixteen
+    const double mine = km == 0 ? v[0] : (km == 1 ? v[1] : (km == 2 ? v[2] : v[3]));
+    const double p = __shfl_sync(0xffffffffu, mine, (threadIdx.x & 16) + (k & 15));
+    if (i == k) {
+      if (q == 0) bad[b] = p > 1e-300 ? 0 : 1;
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {
+        const int j = q + 16 * m;
+        row[b][j] = (j == k ? 1.0 : v[m]) / p;
+      }
+    }
+    if (q == (k & 15)) col[b][i] = mine;
     __syncthreads();
-    const double p = A[k * 64 + k];
-    if (!(p > 1e-300)) {
+    if (bad[b]) {
       if (threadIdx.x == 0) *ok = 0;
       return;
     }
-    if ((int)threadIdx.x < n) colk[threadIdx.x] = A[threadIdx.x * 64 + k];
-    __syncthreads();
-    if ((int)threadIdx.x < n) {
-      const int j = threadIdx.x;
-      A[k * 64 + j] = (j == k ? 1.0 : A[k * 64 + j]) / p;
-    }
-    __syncthreads();
-    for (int t = threadIdx.x; t < n * n; t += blockDim.x) {
-      const int i = t / n, j = t - i * n;
-      if (i == k) continue;
-      A[i * 64 + j] = (j == k ? 0.0 : A[i * 64 + j]) - colk[i] * A[k * 64 + j];
+    const double ci = col[b][i];
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const int j = q + 16 * m;
+      v[m] = i == k ? row[b][j] : (j == k ? 0.0 : v[m]) - ci * row[b][j];
     }
   }
-  __syncthreads();
-  for (int t = threadIdx.x; t < 64 * 64; t += blockDim.x) inv[t] = A[t];
+#pragma unroll
+  for (int m = 0; m < 4; ++m) inv[i * 64 + q + 16 * m] = i < n && q + 16 * m < n ? v[m] : 0.0;
   if (threadIdx.x == 0) *ok = 1;
 }
 
@@ -1399,6 +1417,7 @@ __global__ void __launch_bounds__(1024) kd_coarse_block(DenseSet<T> G, int use_s
 template <class T>
 __global__ void kw_l1(const int* __restrict__ dbl, int nd, const uint16_t* __restrict__ fmask, T* w, size_t ncap1,
                       Params P, double scale) {
+  pdl_entry();
   int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= (int64_t)nd * 64) return;
   int b = dbl[g >> 6];
@@ -1424,6 +1443,7 @@ __global__ void kw_l1(const int* __restrict__ dbl, int nd, const uint16_t* __res
 template <class T, int D>
 __global__ void kw_coarsen(const int* __restrict__ dbl, int nd, const int* __restrict__ bkey, const T* __restrict__ wf,
                            size_t ncapf, T* wc, size_t ncapc, DenseGrid g3, double scale) {
+  pdl_entry();
   constexpr int H = D / 2;
   int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= (int64_t)nd * H * H * H) return;
@@ -1446,6 +1466,7 @@ __global__ void kw_coarsen(const int* __restrict__ dbl, int nd, const int* __res
 
 template <class T, int D>
 __global__ void kw_diag(const int* __restrict__ dbl, int nd, const int* __restrict__ nbr, T* w, size_t ncap) {
+  pdl_entry();
   int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= (int64_t)nd * D * D * D) return;
   int b = dbl[g / (D * D * D)];
@@ -1466,6 +1487,7 @@ __global__ void kw_diag(const int* __restrict__ dbl, int nd, const int* __restri
 
 template <class T>
 __global__ void kwd_coarsen(DView<T> F, DView<T> C, double scale) {
+  pdl_entry();
   int64_t I = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (I >= C.n) return;
   int X = (int)(I % C.nx), Y = (int)((I / C.nx) % C.ny), Z = (int)(I / ((int64_t)C.nx * C.ny));
@@ -1485,6 +1507,7 @@ __global__ void kwd_coarsen(DView<T> F, DView<T> C, double scale) {
 
 template <class T>
 __global__ void kwd_diag(DView<T> L) {
+  pdl_entry();
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= L.n) return;
   int x = (int)(i % L.nx), y = (int)((i / L.nx) % L.ny), z = (int)(i / ((int64_t)L.nx * L.ny));
@@ -1586,20 +1609,20 @@ static int mg_setup_t(Ctx* c) {
   if (!rc) rc = check(cudaMemsetAsync(w2, 0, ncap2 * 6 * sizeof(T), st));
   if (rc) return rc;
   const double sc = c->mg_scale;
-  kw_l1<T><<<g1, 256, 0, st>>>(c->dbl, nd, c->fmask, w1, ncap1, c->dp, sc); MAC_COUNT(c);
-  kw_coarsen<T, 4><<<g2, 256, 0, st>>>(c->dbl, nd, c->bkey, w1, ncap1, w2, ncap2, c->g3, sc); MAC_COUNT(c);
-  kw_coarsen<T, 2><<<g3, 256, 0, st>>>(c->dbl, nd, c->bkey, w2, ncap2, d3.w, (size_t)d3.n, c->g3, sc); MAC_COUNT(c);
+  launch_k(c, kw_l1<T>, g1, 256, 0, c->dbl, nd, c->fmask, w1, ncap1, c->dp, sc); MAC_COUNT(c);
+  launch_k(c, kw_coarsen<T, 4>, g2, 256, 0, c->dbl, nd, c->bkey, w1, ncap1, w2, ncap2, c->g3, sc); MAC_COUNT(c);
+  launch_k(c, kw_coarsen<T, 2>, g3, 256, 0, c->dbl, nd, c->bkey, w2, ncap2, d3.w, (size_t)d3.n, c->g3, sc); MAC_COUNT(c);
   for (int l = 0; l + 1 < c->ndense; ++l) {
     DView<T> F = dview<T>(c, l), C = dview<T>(c, l + 1);
-    kwd_coarsen<T><<<grid_for(C.n, 256), 256, 0, st>>>(F, C, sc); MAC_COUNT(c);
+    launch_k(c, kwd_coarsen<T>, grid_for(C.n, 256), 256, 0, F, C, sc); MAC_COUNT(c);
   }
-  kw_diag<T, 4><<<g1, 256, 0, st>>>(c->dbl, nd, c->nbr, w1, ncap1); MAC_COUNT(c);
-  kw_diag<T, 2><<<g2, 256, 0, st>>>(c->dbl, nd, c->nbr, w2, ncap2); MAC_COUNT(c);
+  launch_k(c, kw_diag<T, 4>, g1, 256, 0, c->dbl, nd, c->nbr, w1, ncap1); MAC_COUNT(c);
+  launch_k(c, kw_diag<T, 2>, g2, 256, 0, c->dbl, nd, c->nbr, w2, ncap2); MAC_COUNT(c);
   for (int l = 0; l < c->ndense; ++l) {
     DView<T> L = dview<T>(c, l);
-    kwd_diag<T><<<grid_for(L.n, 256), 256, 0, st>>>(L); MAC_COUNT(c);
+    launch_k(c, kwd_diag<T>, grid_for(L.n, 256), 256, 0, L); MAC_COUNT(c);
   }
-  kd_coarsest_inverse<T><<<1, 1024, 0, st>>>(dview<T>(c, c->ndense - 1), c->coarse_inv, c->coarse_ok); MAC_COUNT(c);
+  launch_k(c, kd_coarsest_inverse<T>, 1, 1024, 0, dview<T>(c, c->ndense - 1), c->coarse_inv, c->coarse_ok); MAC_COUNT(c);
   return check(cudaGetLastError());
 }
 

@@ -147,6 +147,7 @@ __global__ void __launch_bounds__(512) k_fmask(const int* __restrict__ blist, co
                                                const int* __restrict__ bkey, const int8_t* __restrict__ lay,
                                                const uint8_t* __restrict__ type, const uint8_t* __restrict__ flags,
                                                uint16_t* fmask, int* dbl, Scalars* ds) {
+  pdl_entry();
   __shared__ int64_t sb[6];
   int b = blist[blockIdx.x];
   load_face_bases(nbr, b, sb);
@@ -208,6 +209,7 @@ constexpr int64_t kOrderMaxSlots = (int64_t)1 << 26;  // larger boxes keep the a
 
 __global__ void k_order_scatter(const int* __restrict__ dbl, int nd, const int* __restrict__ bkey, DenseGrid g,
                                 int* __restrict__ map) {
+  pdl_entry();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= nd) return;
   int b = dbl[i];
@@ -216,6 +218,7 @@ __global__ void k_order_scatter(const int* __restrict__ dbl, int nd, const int* 
 
 __global__ void __launch_bounds__(kOrderBlock) k_order_count(const int* __restrict__ map, int64_t n,
                                                              int* __restrict__ cnt) {
+  pdl_entry();
   int64_t i = (int64_t)blockIdx.x * kOrderBlock + threadIdx.x;
   int k = __syncthreads_count(i < n && map[i] >= 0);
   if (threadIdx.x == 0) cnt[blockIdx.x] = k;
@@ -224,6 +227,7 @@ __global__ void __launch_bounds__(kOrderBlock) k_order_count(const int* __restri
 // Exclusive prefix sum of nb block counts in place, one block: each thread
 // sums a contiguous run, the run totals are scanned through shared memory.
 __global__ void __launch_bounds__(kOrderBlock) k_order_scan(int* cnt, int nb) {
+  pdl_entry();
   __shared__ int tot[kOrderBlock];
   const int per = (nb + kOrderBlock - 1) / kOrderBlock;
   const int lo = threadIdx.x * per, hi = min(nb, lo + per);
@@ -247,6 +251,7 @@ __global__ void __launch_bounds__(kOrderBlock) k_order_scan(int* cnt, int nb) {
 
 __global__ void __launch_bounds__(kOrderBlock) k_order_write(const int* __restrict__ map, int64_t n,
                                                              const int* __restrict__ off, int* __restrict__ dbl) {
+  pdl_entry();
   __shared__ int wsum[kOrderBlock / 32];
   int64_t i = (int64_t)blockIdx.x * kOrderBlock + threadIdx.x;
   int b = i < n ? map[i] : -1;
@@ -261,6 +266,7 @@ __global__ void __launch_bounds__(kOrderBlock) k_order_write(const int* __restri
 
 __global__ void k_drow(const int* __restrict__ dbl, int nd, const int* __restrict__ nbr, const int* __restrict__ bkey,
                        DenseGrid g, int* __restrict__ drow) {
+  pdl_entry();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 8 * (int64_t)nd) return;
   const int k = (int)(t & 7);
@@ -311,14 +317,15 @@ static int order_domain_bricks(Ctx* c) {
   cudaStream_t st = c->stream;
   int rc = check(cudaMemsetAsync(c->dbl_map, 0xff, sizeof(int) * n, st));
   if (rc) return rc;
-  k_order_scatter<<<(nd + 255) / 256, 256, 0, st>>>(c->dbl, nd, c->bkey, g, c->dbl_map); MAC_COUNT(c);
-  k_order_count<<<(unsigned)nb, kOrderBlock, 0, st>>>(c->dbl_map, n, c->dbl_cnt); MAC_COUNT(c);
-  k_order_scan<<<1, kOrderBlock, 0, st>>>(c->dbl_cnt, (int)nb); MAC_COUNT(c);
-  k_order_write<<<(unsigned)nb, kOrderBlock, 0, st>>>(c->dbl_map, n, c->dbl_cnt, c->dbl); MAC_COUNT(c);
+  launch_k(c, k_order_scatter, (nd + 255) / 256, 256, 0, c->dbl, nd, c->bkey, g, c->dbl_map); MAC_COUNT(c);
+  launch_k(c, k_order_count, (unsigned)nb, kOrderBlock, 0, c->dbl_map, n, c->dbl_cnt); MAC_COUNT(c);
+  launch_k(c, k_order_scan, 1, kOrderBlock, 0, c->dbl_cnt, (int)nb); MAC_COUNT(c);
+  launch_k(c, k_order_write, (unsigned)nb, kOrderBlock, 0, c->dbl_map, n, c->dbl_cnt, c->dbl); MAC_COUNT(c);
   return check(cudaGetLastError());
 }
 
 __global__ void k_setup_reset(Scalars* ds) {
+  pdl_entry();
   ds->nunknown = 0;
   ds->ndom = 0;
   for (int a = 0; a < 3; ++a) {
@@ -342,6 +349,7 @@ __global__ void __launch_bounds__(512) k_dirichlet(const int* __restrict__ blist
                                                    const double* __restrict__ ux, const double* __restrict__ uy,
                                                    const double* __restrict__ uz, double* __restrict__ pdir,
                                                    Params P) {
+  pdl_entry();
   __shared__ int64_t sb[6];
   int b = blist[blockIdx.x];
   load_face_bases(nbr, b, sb);
@@ -383,6 +391,7 @@ __global__ void __launch_bounds__(kBT) k_divergence(const int* __restrict__ drow
                                                     const double* __restrict__ pres, double* __restrict__ rhs,
                                                     double* __restrict__ x, double* __restrict__ r, int warm,
                                                     double* partial, Params P, const double* __restrict__ pdir) {
+  pdl_entry();
   __shared__ int64_t sb[6];
   const int b = load_drow(drow, sb);
   __syncthreads();
@@ -453,6 +462,7 @@ __global__ void __launch_bounds__(kBT) k_residual(const int* __restrict__ drow,
                                                   const uint16_t* __restrict__ fmask, const double* __restrict__ rhs,
                                                   const double* __restrict__ x, double* __restrict__ r,
                                                   double* partial, Params P) {
+  pdl_entry();
   __shared__ int64_t sb[6];
   const int b = load_drow(drow, sb);
   __syncthreads();
@@ -570,6 +580,7 @@ __global__ void k_fin_rr(const double* partial, int nblk, Scalars* ds, double rt
 }
 
 __global__ void k_fin_bnorm(const double* partial, int nblk, Scalars* ds) {
+  pdl_entry();
   double bb, unused;
   sum_partials(partial, nblk, &bb, &unused);
   if (threadIdx.x == 0) {
@@ -581,6 +592,7 @@ __global__ void k_fin_bnorm(const double* partial, int nblk, Scalars* ds) {
 }
 
 __global__ void k_fin_rr_initial(const double* partial, int nblk, Scalars* ds, double rtol2) {
+  pdl_entry();
   double rr, unused;
   sum_partials(partial, nblk, &rr, &unused);
   if (threadIdx.x == 0) {
@@ -626,7 +638,9 @@ __global__ void __launch_bounds__(512) k_gradient(const int* __restrict__ blist,
                                                   const int8_t* __restrict__ lay, const uint8_t* __restrict__ type,
                                                   const uint8_t* __restrict__ flags, const double* __restrict__ x,
                                                   double* __restrict__ pres, double* ux, double* uy, double* uz,
-                                                  Params P, const double* __restrict__ pdir) {
+                                                  Params P, const double* __restrict__ pdir, Scalars* ds) {
+  pdl_entry();
+  if (blockIdx.x == 0 && threadIdx.x == 0) ds->div_bits = 0;  // for the divergence check
   __shared__ int64_t sb[6];
   int b = blist[blockIdx.x];
   load_face_bases(nbr, b, sb);
@@ -674,6 +688,7 @@ __global__ void __launch_bounds__(kBT) k_divmax(const int* __restrict__ drow,
                                                 const uint16_t* __restrict__ fmask, const double* __restrict__ ux,
                                                 const double* __restrict__ uy, const double* __restrict__ uz, Params P,
                                                 Scalars* ds) {
+  pdl_entry();
   __shared__ int64_t sb[6];
   const int b = load_drow(drow, sb);
   __syncthreads();
@@ -704,8 +719,6 @@ __global__ void __launch_bounds__(kBT) k_divmax(const int* __restrict__ drow,
   for (int s = 16; s > 0; s >>= 1) mx = fmax(mx, __shfl_down_sync(0xffffffffu, mx, s));
   if ((threadIdx.x & 31) == 0) atomicMax(&ds->div_bits, (unsigned long long)__double_as_longlong(mx));
 }
-
-__global__ void k_zero_div(Scalars* ds) { ds->div_bits = 0; }
 
 // ------------------------------------------------------------ drivers
 // ------------------------------------------- learned preconditioner glue
@@ -827,10 +840,11 @@ int learned_precondition(Ctx* c, int first) {
 int setup_system(Ctx* c) {
   cudaStream_t st = c->stream;
   int n = c->nlive_host;
+  c->lag_pending = 0;
   prof_begin(c, PH_SETUP);
-  k_setup_reset<<<1, 1, 0, st>>>(c->ds); MAC_COUNT(c);
+  launch_k(c, k_setup_reset, 1, 1, 0, c->ds); MAC_COUNT(c);
   if (n > 0) {
-    k_fmask<<<n, 512, 0, st>>>(c->blist, c->nbr, c->bkey, c->lay, c->type, c->flags, c->fmask, c->dbl, c->ds); MAC_COUNT(c);
+    launch_k(c, k_fmask, n, 512, 0, c->blist, c->nbr, c->bkey, c->lay, c->type, c->flags, c->fmask, c->dbl, c->ds); MAC_COUNT(c);
   }
   int rc = read_scalars(c);
   if (rc) return rc;
@@ -838,7 +852,7 @@ int setup_system(Ctx* c) {
   c->stats.unknowns = c->hs->nunknown;
   if ((rc = order_domain_bricks(c))) return rc;
   if (c->ndom_host > 0) {
-    k_drow<<<grid_for(8 * (int64_t)c->ndom_host, 256), 256, 0, st>>>(c->dbl, c->ndom_host, c->nbr, c->bkey,
+    launch_k(c, k_drow, dim3(grid_for(8 * (int64_t)c->ndom_host, 256)), 256, 0, c->dbl, c->ndom_host, c->nbr, c->bkey,
                                                                                domain_box(c), c->drow); MAC_COUNT(c);
   }
   if (c->ndom_host > 0 && c->prm.solver != MAC_SOLVER_CG_FP64) {
@@ -865,11 +879,21 @@ void cg_finish_update(Ctx* c) {
            c->prm.max_iters); MAC_COUNT(c);
 }
 
-int project(Ctx* c, int ib) {
+int project(Ctx* c, int ib, int more) {
   size_t cap = (size_t)c->cap_bricks * kCells;
   double* U[3] = {c->f64 + (size_t)(3 * ib) * cap, c->f64 + (size_t)(3 * ib + 1) * cap,
                   c->f64 + (size_t)(3 * ib + 2) * cap};
-  return project_field(c, U, U);
+  return project_field(c, U, U, more);
+}
+
+// Books the outcome of a solve from scalars read back; returns its status.
+static int book_solve(Ctx* c, const Scalars& h) {
+  const double relres = h.bnorm2 > 0 ? sqrt(h.rr / h.bnorm2) : 0.0;
+  c->stats.iterations = h.iters;
+  c->stats.total_iterations += h.iters;
+  c->stats.relres = relres;
+  c->stats.solves += 1;
+  return relres <= c->prm.rtol ? MAC_OK : MAC_ERR_NOT_CONVERGED;
 }
 
 // The projection of vector field U (Divergence_Projection: divergence,
@@ -878,7 +902,7 @@ int project(Ctx* c, int ib) {
 // (Speed_GetRef(-1, false), src/Policy_Dirichlet_Boundary.h:100-102): U
 // itself, except in the force projection of pipeline B
 // (src/Algorithms_Solve_Pressure_Force.h:16-24), where U is the acceleration.
-int project_field(Ctx* c, double* const* U, const double* const* D) {
+int project_field(Ctx* c, double* const* U, const double* const* D, int more) {
   if (!c->system_ready) {
     int rc = setup_system(c);
     if (rc) return rc;
@@ -888,10 +912,12 @@ int project_field(Ctx* c, double* const* U, const double* const* D) {
   size_t cap = (size_t)c->cap_bricks * kCells;
   int status = MAC_OK;
   int rc;
+  bool unread = false;  // the whole solve was enqueued at once: its scalars are read after what follows
+  c->lag_status = MAC_OK;
   // the viscous composition projects with Dirichlet air pressures
   double* pdir = c->dp.nu > 0 ? c->pdir : nullptr;
   if (pdir && nd == 0 && c->nlive_host > 0) {
-    k_dirichlet<<<c->nlive_host, 512, 0, st>>>(c->blist, c->nbr, c->lay, c->type, D[0], D[1], D[2], pdir,
+    launch_k(c, k_dirichlet, c->nlive_host, 512, 0, c->blist, c->nbr, c->lay, c->type, D[0], D[1], D[2], pdir,
                                                c->dp); MAC_COUNT(c);
   }
   if (nd > 0) {
@@ -899,16 +925,16 @@ int project_field(Ctx* c, double* const* U, const double* const* D) {
     double rtol2 = c->prm.rtol * c->prm.rtol;
     prof_begin(c, PH_DIVERGENCE);
     if (pdir) {
-      k_dirichlet<<<c->nlive_host, 512, 0, st>>>(c->blist, c->nbr, c->lay, c->type, D[0], D[1], D[2], pdir,
+      launch_k(c, k_dirichlet, c->nlive_host, 512, 0, c->blist, c->nbr, c->lay, c->type, D[0], D[1], D[2], pdir,
                                                  c->dp); MAC_COUNT(c);
     }
-    k_divergence<<<nd, kBT, 0, st>>>(c->drow, c->fmask, U[0], U[1], U[2], c->f64 + (size_t)PRES * cap, c->b,
+    launch_k(c, k_divergence, nd, kBT, 0, c->drow, c->fmask, U[0], U[1], U[2], c->f64 + (size_t)PRES * cap, c->b,
                                      c->x, c->r, warm, c->partial, c->dp, pdir); MAC_COUNT(c);
     prof_end(c, PH_DIVERGENCE);
-    k_fin_bnorm<<<1, 1024, 0, st>>>(c->partial, nd, c->ds); MAC_COUNT(c);
+    launch_k(c, k_fin_bnorm, 1, 1024, 0, c->partial, nd, c->ds); MAC_COUNT(c);
     if (warm) {
-      k_residual<<<nd, kBT, 0, st>>>(c->drow, c->fmask, c->b, c->x, c->r, c->partial, c->dp); MAC_COUNT(c);
-      k_fin_rr_initial<<<1, 1024, 0, st>>>(c->partial, nd, c->ds, rtol2); MAC_COUNT(c);
+      launch_k(c, k_residual, nd, kBT, 0, c->drow, c->fmask, c->b, c->x, c->r, c->partial, c->dp); MAC_COUNT(c);
+      launch_k(c, k_fin_rr_initial, 1, 1024, 0, c->partial, nd, c->ds, rtol2); MAC_COUNT(c);
     }
     // a step's particle binning runs beside this solve's iterations
     if ((rc = launch_side_binning(c))) return rc;
@@ -945,7 +971,7 @@ int project_field(Ctx* c, double* const* U, const double* const* D) {
         prof_end(c, PH_VCYCLE);
         if (rc) return rc;
         if (resident) {
-          lagged = true;
+          unread = true;
           break;
         }
       }
@@ -1018,19 +1044,14 @@ int project_field(Ctx* c, double* const* U, const double* const* D) {
           // MG-PCG from the current x: true residual, fresh directions
           learned = false;
           c->stats.fallbacks += 1;
-          k_residual<<<nd, kBT, 0, st>>>(c->drow, c->fmask, c->b, c->x, c->r, c->partial, c->dp); MAC_COUNT(c);
-          k_fin_rr_initial<<<1, 1024, 0, st>>>(c->partial, nd, c->ds, rtol2); MAC_COUNT(c);
+          launch_k(c, k_residual, nd, kBT, 0, c->drow, c->fmask, c->b, c->x, c->r, c->partial, c->dp); MAC_COUNT(c);
+          launch_k(c, k_fin_rr_initial, 1, 1024, 0, c->partial, nd, c->ds, rtol2); MAC_COUNT(c);
           first = 1;
         }
       }
     }
     if (lagged && (rc = read_scalars(c))) return rc;
-    double relres = c->hs->bnorm2 > 0 ? sqrt(c->hs->rr / c->hs->bnorm2) : 0.0;
-    c->stats.iterations = c->hs->iters;
-    c->stats.total_iterations += c->hs->iters;
-    c->stats.relres = relres;
-    c->stats.solves += 1;
-    if (!(relres <= c->prm.rtol)) status = MAC_ERR_NOT_CONVERGED;
+    if (!unread) status = book_solve(c, *c->hs);
   } else {
     c->stats.iterations = 0;
     c->stats.relres = 0.0;
@@ -1039,17 +1060,27 @@ int project_field(Ctx* c, double* const* U, const double* const* D) {
   int n = c->nlive_host;
   if (n > 0) {
     prof_begin(c, PH_GRADIENT);
-    k_gradient<<<n, 512, 0, st>>>(c->blist, c->nbr, c->lay, c->type, c->flags, c->x, c->f64 + (size_t)PRES * cap,
-                                  U[0], U[1], U[2], c->dp, pdir); MAC_COUNT(c);
+    launch_k(c, k_gradient, n, 512, 0, c->blist, c->nbr, c->lay, c->type, c->flags, c->x, c->f64 + (size_t)PRES * cap,
+                                  U[0], U[1], U[2], c->dp, pdir, c->ds); MAC_COUNT(c);
     prof_end(c, PH_GRADIENT);
   }
-  if (c->prm.div_check && nd > 0) {
-    k_zero_div<<<1, 1, 0, st>>>(c->ds); MAC_COUNT(c);
-    k_divmax<<<nd, kBT, 0, st>>>(c->drow, c->fmask, U[0], U[1], U[2], c->dp, c->ds); MAC_COUNT(c);
-    rc = read_scalars(c);
+  const bool check_div = c->prm.div_check && nd > 0 && !more;
+  if (check_div) {
+    launch_k(c, k_divmax, nd, kBT, 0, c->drow, c->fmask, U[0], U[1], U[2], c->dp, c->ds); MAC_COUNT(c);
+  }
+  if (unread && more) {
+    rc = check(cudaMemcpyAsync(&c->hs_lag[2], c->ds, sizeof(Scalars), cudaMemcpyDeviceToHost, st));
     if (rc) return rc;
-    unsigned long long bits = c->hs->div_bits;
-    std::memcpy(&c->stats.max_div, &bits, sizeof(double));
+    c->lag_pending = 1;
+  } else if (unread || check_div || c->lag_pending) {
+    if ((rc = read_scalars(c))) return rc;
+    if (c->lag_pending) c->lag_status = book_solve(c, c->hs_lag[2]);
+    c->lag_pending = 0;
+    if (unread) status = book_solve(c, *c->hs);
+    if (check_div) {
+      unsigned long long bits = c->hs->div_bits;
+      std::memcpy(&c->stats.max_div, &bits, sizeof(double));
+    }
   }
   rc = check(cudaGetLastError());
   return rc ? rc : status;

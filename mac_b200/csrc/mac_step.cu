@@ -18,15 +18,20 @@ int rk2tvd(Ctx* c) {
   int rc = setup_system(c);
   if (rc) return rc;
   if ((rc = rk_stage(c, 1))) return rc;
-  int s1 = project(c, 1);
+  // the first projection's outcome is read with the second's where its whole
+  // solve is enqueued at once, and its divergence check is the second's
+  int s1 = project(c, 1, 1);
   if (s1 && s1 != MAC_ERR_NOT_CONVERGED) return s1;
   if ((rc = rk_stage(c, 2))) return rc;
-  int s2 = project(c, 0);
+  int s2 = project(c, 0, 0);
   if (s2) return s2;
-  return s1;
+  return c->lag_status ? c->lag_status : s1;
 }
 
-__global__ void k_advance_time(Scalars* ds) { ds->t += ds->dt; }
+__global__ void k_advance_time(Scalars* ds) {
+  pdl_entry();
+  ds->t += ds->dt;
+}
 
 // Algorithms_RungeKutta_all::Do (src/Algorithms_RungeKutta_all.h:35-156) with
 // the policy of test/Jet3.cpp:642-675: the acceleration is zeroed, then each
@@ -110,7 +115,7 @@ static int step(Ctx* c) {
     rc = move_particles(c);
   }
   if (rc) return rc;
-  k_advance_time<<<1, 1, 0, c->stream>>>(c->ds); MAC_COUNT(c);
+  launch_k(c, k_advance_time, 1, 1, 0, c->ds); MAC_COUNT(c);
   rc = check(cudaGetLastError());
   return rc ? rc : ode;
 }
@@ -630,7 +635,7 @@ int mac_pressure_project(void* ctx, int ispeed) {
   CTX_OR_FAIL();
   if (ispeed < 0 || ispeed > 1) return MAC_ERR_INVALID;
   int rc = mac::setup_system(c);
-  return rc ? rc : mac::project(c, ispeed);
+  return rc ? rc : mac::project(c, ispeed, 0);
 }
 int mac_pressure_init(void* ctx) {
   CTX_OR_FAIL();

@@ -20,7 +20,19 @@
 
 namespace mac {
 
-constexpr int kTopoBlocks = 1184;  // 8 x 148 SMs, grid-stride over bricks
+// The passes are grid-stride loops over the live bricks, whose number the device
+// alone knows: at most 8 blocks an SM, and for small worlds about two a brick of
+// the last count read back (1,184 blocks for 300 bricks cost a microsecond of
+// launch each, a third of such a pass).
+constexpr int kTopoBlocks = 1184;
+static int topo_grid(const Ctx* c) {
+  const int g = 2 * c->nlive_host + 64;
+  return g < kTopoBlocks ? g : kTopoBlocks;
+}
+static int particle_grid(const Ctx* c) {
+  const int64_t g = (c->np_host + 255) / 256 + 16;
+  return (int)(g < 2 * kTopoBlocks ? g : 2 * kTopoBlocks);
+}
 
 // --------------------------------------------------------------- hashing
 __device__ int hash_insert(unsigned long long* hk, int64_t hcap, unsigned long long key, int* newslots,
@@ -45,7 +57,13 @@ __device__ int hash_insert(unsigned long long* hk, int64_t hcap, unsigned long l
   return -1;
 }
 
-__global__ void k_hash_clear(unsigned long long* hk, int* hv, int64_t hcap) {
+// compacted: the live list was compacted by the kernel before (its count becomes the count).
+__global__ void k_hash_clear(unsigned long long* hk, int* hv, int64_t hcap, int compacted, Scalars* ds) {
+  pdl_entry();
+  if (compacted && blockIdx.x == 0 && threadIdx.x == 0) {
+    ds->nlive = ds->nlive_new;
+    ds->nlive_new = 0;
+  }
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < hcap) {
     hk[i] = kEmptyKey;
@@ -55,6 +73,7 @@ __global__ void k_hash_clear(unsigned long long* hk, int* hv, int64_t hcap) {
 
 __global__ void k_hash_insert_live(const int* __restrict__ blist, const int* __restrict__ bkey,
                                    unsigned long long* hk, int* hv, int64_t hcap, Scalars* ds) {
+  pdl_entry();
   int n = ds->nlive;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     int b = blist[i];
@@ -73,9 +92,17 @@ __global__ void k_hash_insert_live(const int* __restrict__ blist, const int* __r
   }
 }
 
+// What k_alloc_bricks' blocks have read by now: the next kernel clears it.
+__device__ inline void after_alloc(Scalars* ds) {
+  if (ds->nfree < 0) ds->nfree = 0;
+  ds->nnew = 0;
+}
+
 __global__ void k_build_nbr(const int* __restrict__ blist, const int* __restrict__ bkey,
                             const unsigned long long* __restrict__ hk, const int* __restrict__ hv,
-                            int64_t hcap, int* __restrict__ nbr, Scalars* ds) {
+                            int64_t hcap, int* __restrict__ nbr, int allocated, Scalars* ds) {
+  pdl_entry();
+  if (allocated && blockIdx.x == 0 && threadIdx.x == 0) after_alloc(ds);
   int n = ds->nlive;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (int64_t)n * kNbr;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -88,24 +115,6 @@ __global__ void k_build_nbr(const int* __restrict__ blist, const int* __restrict
   }
 }
 
-__global__ void k_bbox(const int* __restrict__ blist, const int* __restrict__ bkey, Scalars* ds) {
-  int n = ds->nlive;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    int b = blist[i];
-    for (int a = 0; a < 3; ++a) {
-      atomicMin(&ds->bbox[a], bkey[3 * b + a]);
-      atomicMax(&ds->bbox[3 + a], bkey[3 * b + a]);
-    }
-  }
-}
-
-__global__ void k_bbox_reset(Scalars* ds) {
-  for (int a = 0; a < 3; ++a) {
-    ds->bbox[a] = 0x3fffffff;
-    ds->bbox[3 + a] = -0x3fffffff;
-  }
-}
-
 // New hash slots get a pool brick initialised to the prototype chunk
 // (Data_Chunk::Allocate copies the prototype cell into every slot:
 // src/Data_Chunk_Base.h:20-29, src/Data_Chunk_Speed.h:99-123).
@@ -113,8 +122,10 @@ __global__ void k_alloc_bricks(const int* __restrict__ newslots, const unsigned 
                                int* hv, int* bkey, int* blist, const int* __restrict__ freelist,
                                int8_t* lay, uint8_t* type, uint8_t* flags, double* f64, int16_t* depth,
                                double* u2, size_t cap_cells, int64_t cap_bricks, Scalars* ds) {
+  pdl_entry();
   __shared__ int sb;
   int n = ds->nnew;
+  if (blockIdx.x == 0 && threadIdx.x == 0) ds->done = n > 0 ? 1 : 0;  // whether particle marking has a second pass
   if (n > cap_bricks) n = (int)cap_bricks;
   for (int i = blockIdx.x; i < n; i += gridDim.x) {
     if (threadIdx.x == 0) {
@@ -154,17 +165,13 @@ __global__ void k_alloc_bricks(const int* __restrict__ newslots, const unsigned 
   }
 }
 
-__global__ void k_after_alloc(Scalars* ds) {
-  if (ds->nfree < 0) ds->nfree = 0;
-  ds->nnew = 0;
-}
-
 // ------------------------------------------------- Initialize_MacCell
 // src/Algorithms_Initialize_MacCell.h:15-21: every existing cell -> empty layer.
 // Depth composition (src/Algorithms_Initialize_Layer_And_Depth.h:16-33): also
 // fluid cells that are not interior lose their depth.
 __global__ void k_initialize(const int* __restrict__ blist, int8_t* lay, const uint8_t* __restrict__ type,
                              int16_t* depth, Scalars* ds) {
+  pdl_entry();
   int n = ds->nlive;
   for (int bi = blockIdx.x; bi < n; bi += gridDim.x) {
     size_t base = (size_t)blist[bi] * kCells;
@@ -193,6 +200,8 @@ __global__ void k_mark_particles(const double* __restrict__ px, const double* __
                                  const double* __restrict__ pz, Params P, unsigned long long* hk, int* hv,
                                  int64_t hcap, int* newslots, int64_t cap_new, int8_t* lay, uint8_t* type,
                                  const int16_t* __restrict__ depth, uint8_t* pkeep, Scalars* ds, int pass) {
+  pdl_entry();
+  if (pass == 1 && blockIdx.x == 0 && threadIdx.x == 0) after_alloc(ds);
   if (pass == 1 && ds->done == 0) return;  // no brick was missing in pass 0
   int64_t n = ds->np;
   for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
@@ -232,6 +241,7 @@ struct PartMove {
 };
 
 __global__ void k_compact_particles(PartMove M, const uint8_t* __restrict__ pkeep, Scalars* ds) {
+  pdl_entry();
   const int64_t n = ds->np;
   const int lane = threadIdx.x & 31;
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += (int64_t)gridDim.x * blockDim.x) {
@@ -249,17 +259,16 @@ __global__ void k_compact_particles(PartMove M, const uint8_t* __restrict__ pkee
 }
 
 __global__ void k_compact_particles_done(Scalars* ds) {
+  pdl_entry();
   ds->np = (int64_t)ds->np_new;
   ds->np_new = 0;
 }
 
-// Remembers across the alloc kernel whether pass 1 of the particle marking must run.
-__global__ void k_note_missing(Scalars* ds) { ds->done = ds->nnew > 0 ? 1 : 0; }
-__global__ void k_clear_note(Scalars* ds) { ds->done = 0; }
-
 // ------------------------------------------------ Create_Fluid_Particle
 // Same jitter as the oracle's restatement: splitmix64 over (seed, key, slot, axis).
 __device__ inline unsigned long long mix64(unsigned long long z) {
+  pdl_entry();
+  pdl_entry();
   z += 0x9E3779B97F4A7C15ull;
   z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
   z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
@@ -297,6 +306,7 @@ __global__ void k_refill(const int* __restrict__ blist, const int* __restrict__ 
                          const uint8_t* __restrict__ type, const int16_t* __restrict__ depth, double* px,
                          double* py, double* pz, int64_t cap_particles, unsigned long long seed, Params P,
                          Scalars* ds, int no_particles) {
+  pdl_entry();
   int n = ds->nlive;
   const int side = 2 * P.refill_cube + 1;
   const int per = P.refill_cube > 0 ? side * side * side : 8;
@@ -361,6 +371,7 @@ __global__ void k_refill(const int* __restrict__ blist, const int* __restrict__ 
 __global__ void k_dilate(const int* __restrict__ blist, const int* __restrict__ bkey,
                          const int8_t* __restrict__ lay, unsigned long long* hk, const int* hv, int64_t hcap,
                          int* newslots, int64_t cap_new, int R, Scalars* ds) {
+  pdl_entry();
   __shared__ int any0;
   int n = ds->nlive;
   for (int bi = blockIdx.x; bi < n; bi += gridDim.x) {
@@ -402,6 +413,7 @@ __device__ inline int8_t lay_at(const int8_t* __restrict__ lay, const int* __res
 // (src/Data_CellType_Fluid_Air_Solid_Inflow_Interior_0_Pres.tpp:217-223).
 __global__ void k_bfs_level(const int* __restrict__ blist, const int* __restrict__ nbr, int8_t* lay,
                             uint8_t* type, int L, int ring, Scalars* ds) {
+  pdl_entry();
   int n = ds->nlive;
   for (int bi = blockIdx.x; bi < n; bi += gridDim.x) {
     int b = blist[bi];
@@ -440,6 +452,7 @@ __global__ void k_bfs_level(const int* __restrict__ blist, const int* __restrict
 // inward BFS of :104-134.
 __global__ void k_depth_seed(const int* __restrict__ blist, const int* __restrict__ nbr,
                              const int8_t* __restrict__ lay, int16_t* depth, Scalars* ds) {
+  pdl_entry();
   int n = ds->nlive;
   for (int bi = blockIdx.x; bi < n; bi += gridDim.x) {
     int b = blist[bi];
@@ -473,8 +486,13 @@ __global__ void k_depth_seed(const int* __restrict__ blist, const int* __restric
 constexpr int16_t kDepthInf = 0x7fff;
 constexpr int16_t kDepthNone = -2;
 
+// The launches of a batch know of each other: launch `it` does nothing when the
+// one before it changed nothing.
 __global__ void __launch_bounds__(512) k_depth_relax(const int* __restrict__ blist, const int* __restrict__ nbr,
-                                                     const int8_t* __restrict__ lay, int16_t* depth, Scalars* ds) {
+                                                     const int8_t* __restrict__ lay, int16_t* depth, int it,
+                                                     Scalars* ds) {
+  pdl_entry();
+  if (it > 0 && ds->dchanged[it - 1] == 0) return;
   __shared__ int16_t sd[1000];  // 10^3 with halo: kDepthNone off the layer-0 set, kDepthInf unreached
   int n = ds->nlive;
   const int t = threadIdx.x;
@@ -518,19 +536,19 @@ __global__ void __launch_bounds__(512) k_depth_relax(const int* __restrict__ bli
     }
     if (part && cur < start) {
       depth[(size_t)b * kCells + t] = cur;
-      ds->dchanged = 1;
+      ds->dchanged[it] = 1;
     }
     __syncthreads();
   }
 }
-
-__global__ void k_depth_flag_clear(Scalars* ds) { ds->dchanged = 0; }
 
 // Materials of :117-124: a layer-0 cell reached at depth d >= 1 becomes fluid
 // (SetFluid: from air or interior) when d < DepthInterior and interior
 // (SetInterior: always) otherwise; the seeds keep their material.
 __global__ void k_depth_types(const int* __restrict__ blist, const int8_t* __restrict__ lay,
                               const int16_t* __restrict__ depth, uint8_t* type, Params P, Scalars* ds) {
+  pdl_entry();
+  pdl_entry();
   int n = ds->nlive;
   for (int bi = blockIdx.x; bi < n; bi += gridDim.x) {
     size_t base = (size_t)blist[bi] * kCells;
@@ -555,6 +573,7 @@ __global__ void k_depth_types(const int* __restrict__ blist, const int8_t* __res
 // (src/ChunkHashTable.tpp:132-147).
 __global__ void k_delete(const int* __restrict__ blist, int8_t* lay, const uint8_t* __restrict__ flags,
                          uint8_t* alive, Scalars* ds) {
+  pdl_entry();
   __shared__ int any;
   int n = ds->nlive;
   for (int bi = blockIdx.x; bi < n; bi += gridDim.x) {
@@ -580,17 +599,13 @@ __global__ void k_delete(const int* __restrict__ blist, int8_t* lay, const uint8
 
 __global__ void k_compact(const int* __restrict__ blist, int* blist2, int* freelist, const uint8_t* alive,
                           Scalars* ds) {
+  pdl_entry();
   int n = ds->nlive;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     int b = blist[i];
     if (alive[b]) blist2[atomicAdd(&ds->nlive_new, 1)] = b;
     else freelist[atomicAdd(&ds->nfree, 1)] = b;
   }
-}
-
-__global__ void k_compact_done(Scalars* ds) {
-  ds->nlive = ds->nlive_new;
-  ds->nlive_new = 0;
 }
 
 // ------------------------------------------------ Calculate_Time_Step
@@ -601,8 +616,10 @@ __global__ void k_compact_done(Scalars* ds) {
 __global__ void k_cfl(const int* __restrict__ blist, const int8_t* __restrict__ lay,
                       const uint8_t* __restrict__ type, const double* __restrict__ ux,
                       const double* __restrict__ uy, const double* __restrict__ uz, Params P, Scalars* ds) {
+  pdl_entry();
   __shared__ unsigned long long smax;
   __shared__ int scount;
+  __shared__ int last;
   int n = ds->nlive;
   double mx = 0;
   int cnt = 0;
@@ -632,64 +649,58 @@ __global__ void k_cfl(const int* __restrict__ blist, const int8_t* __restrict__ 
   __syncthreads();
   if (threadIdx.x == 0) {
     atomicMax(&ds->cfl_bits, smax);
-    atomicAdd((unsigned long long*)&ds->nfluid, (unsigned long long)scount);
+    atomicAdd((unsigned long long*)&ds->cfl_count, (unsigned long long)scount);
+    __threadfence();
+    last = atomicAdd(&ds->cfl_blocks, 1) == (int)gridDim.x - 1;
   }
-}
-
-__global__ void k_cfl_reset(Scalars* ds) {
-  ds->cfl_bits = 0;
-  ds->nfluid = 0;
-}
-
-__global__ void k_dt_finalize(Params P, Scalars* ds) {
-  double mx = __longlong_as_double((long long)ds->cfl_bits);
-  double dt = 1 / sqrt(mx) * P.cfl;
+  __syncthreads();
+  if (!last || threadIdx.x != 0) return;
+  // the last block: dt from the maximum, and the sums cleared for the next call
+  __threadfence();
+  const double top = __longlong_as_double((long long)atomicExch(&ds->cfl_bits, 0ull));
+  ds->nfluid = (int64_t)atomicExch((unsigned long long*)&ds->cfl_count, 0ull);
+  ds->cfl_blocks = 0;
+  double dt = 1 / sqrt(top) * P.cfl;
   if (dt < P.dt_min) dt = P.dt_min;
   else if (dt > P.dt_max) dt = P.dt_max;
   ds->dt = dt;
 }
 
 // ------------------------------------------------------------ drivers
-int rebuild_index(Ctx* c) {
-  cudaStream_t st = c->stream;
-  k_hash_clear<<<grid_for(c->hcap, 256), 256, 0, st>>>(c->hkeys, c->hval, c->hcap); MAC_COUNT(c);
-  k_hash_insert_live<<<kTopoBlocks, 256, 0, st>>>(c->blist, c->bkey, c->hkeys, c->hval, c->hcap, c->ds); MAC_COUNT(c);
-  k_build_nbr<<<kTopoBlocks, 256, 0, st>>>(c->blist, c->bkey, c->hkeys, c->hval, c->hcap, c->nbr, c->ds); MAC_COUNT(c);
+static int rebuild_index_of(Ctx* c, int compacted) {
+  launch_k(c, k_hash_clear, grid_for(c->hcap, 256), 256, 0, c->hkeys, c->hval, c->hcap, compacted, c->ds); MAC_COUNT(c);
+  launch_k(c, k_hash_insert_live, topo_grid(c), 256, 0, c->blist, c->bkey, c->hkeys, c->hval, c->hcap, c->ds); MAC_COUNT(c);
+  launch_k(c, k_build_nbr, topo_grid(c), 256, 0, c->blist, c->bkey, c->hkeys, c->hval, c->hcap, c->nbr, 0, c->ds); MAC_COUNT(c);
   c->system_ready = false;
   return check(cudaGetLastError());
 }
+int rebuild_index(Ctx* c) { return rebuild_index_of(c, 0); }
 
 static void alloc_new(Ctx* c) {
-  cudaStream_t st = c->stream;
-  k_alloc_bricks<<<kTopoBlocks, 256, 0, st>>>(c->newslots, c->hkeys, c->hval, c->bkey, c->blist, c->freelist,
+  launch_k(c, k_alloc_bricks, topo_grid(c), 256, 0, c->newslots, c->hkeys, c->hval, c->bkey, c->blist, c->freelist,
                                                c->lay, c->type, c->flags, c->f64, c->depth, c->u2,
                                                (size_t)c->cap_bricks * kCells, c->cap_bricks, c->ds); MAC_COUNT(c);
 }
 
 int topo_initialize(Ctx* c) {
-  k_initialize<<<kTopoBlocks, 256, 0, c->stream>>>(c->blist, c->lay, c->type, c->dp.depth_mode ? c->depth : nullptr,
+  launch_k(c, k_initialize, topo_grid(c), 256, 0, c->blist, c->lay, c->type, c->dp.depth_mode ? c->depth : nullptr,
                                                    c->ds); MAC_COUNT(c);
   return check(cudaGetLastError());
 }
 
 int topo_layer_initial(Ctx* c) {
-  cudaStream_t st = c->stream;
-  int g = kTopoBlocks * 2;
-  k_clear_note<<<1, 1, 0, st>>>(c->ds); MAC_COUNT(c);
+  const int g = particle_grid(c);
   uint8_t* keep = c->dp.depth_mode ? c->pkeep : nullptr;
   // the position the topology reads (Data_Particle::imove_particle): 0, or 2
   // during pipeline B's stages 2-4
   const double* kx = c->imove == 2 ? c->pbuf[1][0] : c->px;
   const double* ky = c->imove == 2 ? c->pbuf[1][1] : c->py;
   const double* kz = c->imove == 2 ? c->pbuf[1][2] : c->pz;
-  k_mark_particles<<<g, 256, 0, st>>>(kx, ky, kz, c->dp, c->hkeys, c->hval, c->hcap, c->newslots,
+  launch_k(c, k_mark_particles, g, 256, 0, kx, ky, kz, c->dp, c->hkeys, c->hval, c->hcap, c->newslots,
                                       c->cap_bricks, c->lay, c->type, c->depth, keep, c->ds, 0); MAC_COUNT(c);
-  k_note_missing<<<1, 1, 0, st>>>(c->ds); MAC_COUNT(c);
   alloc_new(c);
-  k_after_alloc<<<1, 1, 0, st>>>(c->ds); MAC_COUNT(c);
-  k_mark_particles<<<g, 256, 0, st>>>(kx, ky, kz, c->dp, c->hkeys, c->hval, c->hcap, c->newslots,
+  launch_k(c, k_mark_particles, g, 256, 0, kx, ky, kz, c->dp, c->hkeys, c->hval, c->hcap, c->newslots,
                                       c->cap_bricks, c->lay, c->type, c->depth, keep, c->ds, 1); MAC_COUNT(c);
-  k_clear_note<<<1, 1, 0, st>>>(c->ds); MAC_COUNT(c);
   if (keep) {
     PartMove M;
     M.src[0] = c->px; M.src[1] = c->py; M.src[2] = c->pz;
@@ -703,8 +714,8 @@ int topo_layer_initial(Ctx* c) {
         }
       M.n = 9;
     }
-    k_compact_particles<<<g, 256, 0, st>>>(M, keep, c->ds); MAC_COUNT(c);
-    k_compact_particles_done<<<1, 1, 0, st>>>(c->ds); MAC_COUNT(c);
+    launch_k(c, k_compact_particles, g, 256, 0, M, keep, c->ds); MAC_COUNT(c);
+    launch_k(c, k_compact_particles_done, 1, 1, 0, c->ds); MAC_COUNT(c);
     std::swap(c->px, c->px2);
     std::swap(c->py, c->py2);
     std::swap(c->pz, c->pz2);
@@ -717,45 +728,45 @@ int topo_layer_initial(Ctx* c) {
 }
 
 int topo_create_fluid(Ctx* c) {
-  k_refill<<<kTopoBlocks, 256, 0, c->stream>>>(c->blist, c->bkey, c->lay, c->type, c->depth, c->px, c->py, c->pz,
+  launch_k(c, k_refill, topo_grid(c), 256, 0, c->blist, c->bkey, c->lay, c->type, c->depth, c->px, c->py, c->pz,
                                                 c->cap_particles, (unsigned long long)c->seed, c->dp, c->ds, 0); MAC_COUNT(c);
   return check(cudaGetLastError());
 }
 
-// Relaxation launches until no depth changes; each launch carries the front at
-// least one brick further, so the bound below (the pool's brick count) is
-// never reached by a valid world.
+// Relaxation launches until no depth changes, in batches between two reads of
+// their marks; each launch carries the front at least one brick further, so the
+// bound below (the pool's brick count) is never reached by a valid world.
 static int depth_bfs(Ctx* c) {
-  cudaStream_t st = c->stream;
   const int limit = (int)(c->cap_bricks < 1000000 ? c->cap_bricks : 1000000) + 2;
-  for (int it = 0;; ++it) {
+  for (int it = 0;; it += kDepthBatch) {
     if (it >= limit) return MAC_ERR_TIMEOUT;
-    k_depth_flag_clear<<<1, 1, 0, st>>>(c->ds); MAC_COUNT(c);
-    k_depth_relax<<<kTopoBlocks, 512, 0, st>>>(c->blist, c->nbr, c->lay, c->depth, c->ds); MAC_COUNT(c);
-    int rc = read_scalars(c);
+    int rc = check(cudaMemsetAsync(c->ds->dchanged, 0, sizeof(c->hs->dchanged), c->stream));
     if (rc) return rc;
-    if (!c->hs->dchanged) break;
+    for (int k = 0; k < kDepthBatch; ++k) {
+      launch_k(c, k_depth_relax, topo_grid(c), 512, 0, c->blist, c->nbr, c->lay, c->depth, k, c->ds); MAC_COUNT(c);
+    }
+    if ((rc = read_scalars(c))) return rc;
+    if (!c->hs->dchanged[kDepthBatch - 1]) break;
   }
-  k_depth_types<<<kTopoBlocks, 256, 0, st>>>(c->blist, c->lay, c->depth, c->type, c->dp, c->ds); MAC_COUNT(c);
+  launch_k(c, k_depth_types, topo_grid(c), 256, 0, c->blist, c->lay, c->depth, c->type, c->dp, c->ds); MAC_COUNT(c);
   return check(cudaGetLastError());
 }
 
 int topo_update_layer(Ctx* c) {
-  cudaStream_t st = c->stream;
   int R = (c->dp.layer_max + 1 + 7) / 8;
   if (R < 1) R = 1;
-  k_dilate<<<kTopoBlocks, 256, 0, st>>>(c->blist, c->bkey, c->lay, c->hkeys, c->hval, c->hcap, c->newslots,
+  launch_k(c, k_dilate, topo_grid(c), 256, 0, c->blist, c->bkey, c->lay, c->hkeys, c->hval, c->hcap, c->newslots,
                                          c->cap_bricks, R, c->ds); MAC_COUNT(c);
   alloc_new(c);
-  k_after_alloc<<<1, 1, 0, st>>>(c->ds); MAC_COUNT(c);
-  k_build_nbr<<<kTopoBlocks, 256, 0, st>>>(c->blist, c->bkey, c->hkeys, c->hval, c->hcap, c->nbr, c->ds); MAC_COUNT(c);
+  launch_k(c, k_build_nbr, topo_grid(c), 256, 0, c->blist, c->bkey, c->hkeys, c->hval, c->hcap, c->nbr, 1,
+           c->ds); MAC_COUNT(c);
   if (c->dp.depth_mode) {
-    k_depth_seed<<<kTopoBlocks, 256, 0, st>>>(c->blist, c->nbr, c->lay, c->depth, c->ds); MAC_COUNT(c);
+    launch_k(c, k_depth_seed, topo_grid(c), 256, 0, c->blist, c->nbr, c->lay, c->depth, c->ds); MAC_COUNT(c);
   }
   for (int L = 1; L <= c->dp.layer_max; ++L) {
-    k_bfs_level<<<kTopoBlocks, 256, 0, st>>>(c->blist, c->nbr, c->lay, c->type, L, 0, c->ds); MAC_COUNT(c);
+    launch_k(c, k_bfs_level, topo_grid(c), 256, 0, c->blist, c->nbr, c->lay, c->type, L, 0, c->ds); MAC_COUNT(c);
   }
-  k_bfs_level<<<kTopoBlocks, 256, 0, st>>>(c->blist, c->nbr, c->lay, c->type, c->dp.layer_max + 1, 1, c->ds); MAC_COUNT(c);
+  launch_k(c, k_bfs_level, topo_grid(c), 256, 0, c->blist, c->nbr, c->lay, c->type, c->dp.layer_max + 1, 1, c->ds); MAC_COUNT(c);
   c->system_ready = false;
   if (c->dp.depth_mode) {
     int rc = depth_bfs(c);
@@ -765,24 +776,19 @@ int topo_update_layer(Ctx* c) {
 }
 
 int topo_delete(Ctx* c) {
-  cudaStream_t st = c->stream;
-  k_delete<<<kTopoBlocks, 256, 0, st>>>(c->blist, c->lay, c->flags, c->alive, c->ds); MAC_COUNT(c);
-  k_compact<<<kTopoBlocks, 256, 0, st>>>(c->blist, c->blist2, c->freelist, c->alive, c->ds); MAC_COUNT(c);
-  k_compact_done<<<1, 1, 0, st>>>(c->ds); MAC_COUNT(c);
+  launch_k(c, k_delete, topo_grid(c), 256, 0, c->blist, c->lay, c->flags, c->alive, c->ds); MAC_COUNT(c);
+  launch_k(c, k_compact, topo_grid(c), 256, 0, c->blist, c->blist2, c->freelist, c->alive, c->ds); MAC_COUNT(c);
   int* t = c->blist;
   c->blist = c->blist2;
   c->blist2 = t;
   c->system_ready = false;
-  return rebuild_index(c);
+  return rebuild_index_of(c, 1);
 }
 
 int topo_dt(Ctx* c) {
-  cudaStream_t st = c->stream;
   size_t cap = (size_t)c->cap_bricks * kCells;
-  k_cfl_reset<<<1, 1, 0, st>>>(c->ds); MAC_COUNT(c);
-  k_cfl<<<kTopoBlocks, 256, 0, st>>>(c->blist, c->lay, c->type, c->f64 + U0X * cap, c->f64 + U0Y * cap,
+  launch_k(c, k_cfl, topo_grid(c), 256, 0, c->blist, c->lay, c->type, c->f64 + U0X * cap, c->f64 + U0Y * cap,
                                       c->f64 + U0Z * cap, c->dp, c->ds); MAC_COUNT(c);
-  k_dt_finalize<<<1, 1, 0, st>>>(c->dp, c->ds); MAC_COUNT(c);
   return check(cudaGetLastError());
 }
 
@@ -799,7 +805,7 @@ int topology_stage(Ctx* c) {
   prof_begin(c, PH_TOPOLOGY);
   if ((rc = topo_initialize(c))) return rc;
   if ((rc = topo_layer_initial(c))) return rc;
-  k_refill<<<kTopoBlocks, 256, 0, c->stream>>>(c->blist, c->bkey, c->lay, c->type, c->depth, c->px, c->py, c->pz,
+  launch_k(c, k_refill, topo_grid(c), 256, 0, c->blist, c->bkey, c->lay, c->type, c->depth, c->px, c->py, c->pz,
                                                 c->cap_particles, (unsigned long long)c->seed, c->dp, c->ds, 1); MAC_COUNT(c);
   if ((rc = topo_update_layer(c))) return rc;
   if ((rc = topo_delete(c))) return rc;
