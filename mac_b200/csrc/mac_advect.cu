@@ -337,8 +337,9 @@ __global__ void __launch_bounds__(256) k_extrapolate(const int* __restrict__ bli
         // Term k of the reference's sum, axis j = k / 2, sign s: a face whose
         // layers and speed are loaded with all others before any is tested (a
         // face waited on up to six dependent rounds, most of a small level's
-        // time: a 32 x 32 x 24 jet's step 1.05 -> 1.03 ms, a force-projection
-        // step of 45 levels 5% less, 29,000 bricks unchanged). j == i, s < 0: the face behind A, valid when A is; its own test
+        // time: a 32 x 32 x 64 jet's step 1.05 -> 1.03 ms, a force-projection
+        // step of 45 levels 5% less, 29,000 bricks unchanged). j == i, s < 0: the
+        // face behind A, valid when A is; its own test
         // layer is that of c - 2 e_i.
         int64_t at[6];
         int8_t l0[6], l1[6];

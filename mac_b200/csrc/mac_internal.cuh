@@ -210,6 +210,7 @@ struct Ctx {
   int res_cluster = 0;        // one cluster of 16 of its blocks fits
   int bulk_grid = 0;          // its grid (blocks resident on all SMs at once)
   int npart_head = 0;         // partial sums the V-cycle's first kernel left (its grid)
+  int npart_tail = 0;         // and its last
   // learned preconditioner (flexible CG): the network and the previous z
   void* unet = nullptr;
   double* zold = nullptr;
@@ -482,21 +483,6 @@ __device__ inline HaloSlot halo_slot(int a) {
   return h;
 }
 
-// The same staging of a plain array: the brick's own 512 cells with 16-byte
-// vector loads (thread t takes cells 4t..4t+3, half a row), the face halos
-// with scalar loads; the values land in s converted to its element type S.
-template <class V>
-__device__ inline void load4(const double* p, V* v) {
-  const double2 a = *reinterpret_cast<const double2*>(p);
-  const double2 c = *reinterpret_cast<const double2*>(p + 2);
-  v[0] = (V)a.x; v[1] = (V)a.y; v[2] = (V)c.x; v[3] = (V)c.y;
-}
-template <class V>
-__device__ inline void load4(const float* p, V* v) {
-  const float4 a = *reinterpret_cast<const float4*>(p);
-  v[0] = (V)a.x; v[1] = (V)a.y; v[2] = (V)a.z; v[3] = (V)a.w;
-}
-
 // Stencil passes over a staged brick give thread t the z-run of four cells
 // (t & 63) + 256 (t >> 6) + 64 k, k = 0..3, of one (x, y) column: the loads
 // and stores of each k stay coalesced, and a cell's z neighbours inside the
@@ -525,18 +511,6 @@ __device__ inline void stage_h1_halo(S* s, const int64_t* sb, F val) {
   }
 #pragma unroll
   for (int a = 0; a < 3; ++a) s[hs[a]] = hv[a];
-}
-
-template <class S, class T>
-__device__ inline void stage_arr(S* s, const T* __restrict__ a, int b, const int64_t* sb) {
-  static_assert(kBT * 4 == kCells, "one 4-cell vector per thread");
-  const int o = 4 * threadIdx.x;
-  S v[4];
-  load4(a + (int64_t)b * kCells + o, v);
-  stage_h1_halo(s, sb, [&](int64_t i) { return a[i]; });
-  const int si = s1_of(o);
-#pragma unroll
-  for (int q = 0; q < 4; ++q) s[si + q] = v[q];
 }
 
 // Kernels of an iterative solve that the host enqueues ahead of its

@@ -21,6 +21,7 @@
 #include <utility>
 
 #include "mac_internal.cuh"
+#include "mac_half.cuh"
 
 namespace mac {
 
@@ -66,228 +67,104 @@ __device__ inline void coords3(int64_t i, int nx, int ny, int64_t n, int& x, int
 }
 
 // ---------------------------------------------------------------- level 0
-// The level-0 sweeps wait mostly on memory latency; in the FP32 form their
-// register caps let 16 blocks of 128 threads share an SM without spills (the
-// FP64 pre-sweep takes 12; the FP64 post-sweeps would spill under any cap).
+// The two-sweep form takes a brick as two half bricks of one warp each
+// (mac_half.cuh), four bricks a block; what a thread may load before the wait
+// on the previous kernel (static data, and what was written two or more
+// launches back) it loads there. They are bound by memory bandwidth now.
+// Measured at 8.0 million unknowns (FP32 levels), before (a 10^3 array in
+// shared memory) and after, us: pre 89.7 and 83.9, restriction 35.4 and 30.2,
+// post 39.4 and 31.3, 40.4 and 34.2, direction and product 70.8 and 52.8.
+//
 // Two Jacobi sweeps from zero, fused: e1 = w D^-1 r, e = e1 + w D^-1 (r - M e1)
 // = w D^-1 ((2 - w) r + sum_f ih2_f e1(n_f)).
 // With update (every CG iteration but the first) the kernel first finishes
 // the previous iteration over all cells of the brick: x += alpha p and
 // r = rin - alpha q into rout with the block's partial r.r. rout is not rin,
-// so a block staging its face halos reads the old r of its neighbours and
-// forms their new r on the fly with the same expression.
+// so a warp reading its halo reads the old r of its neighbours and forms their
+// new r on the fly with the same expression.
 template <class T>
-__global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 16 : 12) k0_pre(const int* __restrict__ drow,
+__global__ void __launch_bounds__(kHT) k0_pre(const int* __restrict__ drow, int nd,
                                               const uint16_t* __restrict__ fmask, const double* __restrict__ rin,
                                               double* __restrict__ rout, double* __restrict__ x,
                                               const double* __restrict__ p, const double* __restrict__ q,
                                               double* partial, const Scalars* ds, int update, T* __restrict__ e,
                                               Params P) {
-  __shared__ int64_t sb[6];
-  __shared__ T sr[kS1];  // w D^-1 r of the brick and its face halo
-  const T om = (T)P.mgw1, om2 = (T)P.mgw2, c0 = (T)(P.mgw1 + P.mgw2 - P.mgw1 * P.mgw2);
-  const T ih2[3] = {(T)P.ih2[0], (T)P.ih2[1], (T)P.ih2[2]};
-  // prologue (static): brick, face neighbours, face masks; each thread takes
-  // the z-run of four cells ob + 64 k (its z neighbours' staged values then
-  // come from registers in the stencil pass)
-  const int b = load_drow(drow, sb);
-  const int ob = zrun_base();
-  uint16_t mk[kCPT];
-#pragma unroll
-  for (int k = 0; k < kCPT; ++k) mk[k] = fmask[(int64_t)b * kCells + ob + 64 * k];
+  const int j = blockIdx.x * kHB + (threadIdx.x >> 6), h = (threadIdx.x >> 5) & 1;
+  Half s;
+  uint32_t mk[4];
+  if (j < nd) {
+    half_load(drow + 8 * (size_t)j, h, s);
+    half_masks(fmask, s, mk);
+  }
   pdl_entry();
   if (solve_done(&ds->done)) return;
   const double al = update ? ds->alpha : 0.0;
-  const int si0 = s1_of(ob);
-  double rv[kCPT];
-  T srv[kCPT];
   double rr = 0;
-#pragma unroll
-  for (int k = 0; k < kCPT; ++k) {
-    const int64_t c = (int64_t)b * kCells + ob + 64 * k;
-    double v = rin[c];
-    if (update) {
-      v = v - al * q[c];
-      rout[c] = v;
-      x[c] += al * p[c];
-      rr += v * v;
-    }
-    rv[k] = v;
-    srv[k] = om * (T)P.dtab[active_index(mk[k])] * (T)v;
-    sr[si0 + 100 * k] = srv[k];
-  }
-  __syncthreads();
-  stage_h1_halo(sr, sb, [&](int64_t i) {
-    const double v = update ? rin[i] - al * q[i] : rin[i];
-    return om * (T)P.dtab[active_index(fmask[i])] * (T)v;
-  });
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < kCPT; ++k) {
-    const int64_t c = (int64_t)b * kCells + ob + 64 * k;
-    const uint16_t m = mk[k];
-    T out = 0;
-    if (m & kDomainBit) {
-      const int si = si0 + 100 * k;
-      const T dinv = (T)P.dtab[active_index(m)];
-      T s = 0;
-#pragma unroll
-      for (int f = 0; f < 6; ++f)
-        if (m & (1u << f)) s += ih2[f >> 1] * zrun_nbr(sr, srv, si, k, f);
-      out = dinv * (c0 * (T)rv[k] + om2 * s);
-    }
-    e[c] = out;
-  }
-  if (update) block_sum<kBT>(rr, 0.0, partial);
+  if (j < nd)
+    rr = half_pre<T>(s, mk, fmask, [&](uint16_t m) { return (T)P.dtab[active_index(m)]; }, P, rin, rout, x, p, q, al,
+                     update, e);
+  if (update) block_sum<kHT>(rr, 0.0, partial);
 }
 
-// res = r - M e on the brick, summed over 2x2x2 children into level 1.
+// res = r - M e on the brick, summed over 2x2x2 children into level 1. r was
+// written by the V-cycle's first kernel, two launches back.
 template <class T>
-__global__ void __launch_bounds__(kBT) k0_restrict(const int* __restrict__ drow,
+__global__ void __launch_bounds__(kHT) k0_restrict(const int* __restrict__ drow, int nd,
                                                    const uint16_t* __restrict__ fmask, const double* __restrict__ r,
                                                    const T* __restrict__ e, T* __restrict__ r1, Params P,
                                                    const int32_t* __restrict__ done) {
-  __shared__ int64_t sb[6];
-  __shared__ T se[kS1];
-  const T ih2[3] = {(T)P.ih2[0], (T)P.ih2[1], (T)P.ih2[2]};
-  // prologue: brick, face neighbours, face masks (static) and r (written by
-  // the V-cycle's first kernel, two launches back)
-  const int b = load_drow(drow, sb);
-  // the stencil pass takes a z-run of four cells of one column per thread
-  // (cells zrun_base() + 64 k): z neighbours inside the run from registers
-  const int ob = zrun_base();
-  uint16_t mk[kCPT];
-  double rk[kCPT];
+  const int j = blockIdx.x * kHB + (threadIdx.x >> 6), h = (threadIdx.x >> 5) & 1;
+  Half s;
+  uint32_t mk[4];
+  double rk[4][2];
+  if (j < nd) {
+    half_load(drow + 8 * (size_t)j, h, s);
+    half_masks(fmask, s, mk);
 #pragma unroll
-  for (int k = 0; k < kCPT; ++k) {
-    const int64_t c = (int64_t)b * kCells + ob + 64 * k;
-    mk[k] = fmask[c];
-    rk[k] = r[c];
+    for (int k = 0; k < 4; ++k) ld2(r + s.c + 64 * k, rk[k]);
   }
   pdl_entry();
-  if (solve_done(done)) return;
-  __syncthreads();
-  stage_arr(se, e, b, sb);
-  __syncthreads();
-  const int si0 = s1_of(ob);
-  T ecs[kCPT];
-#pragma unroll
-  for (int k = 0; k < kCPT; ++k) ecs[k] = se[si0 + 100 * k];
-  T v[kCPT];
-#pragma unroll
-  for (int k = 0; k < kCPT; ++k) {
-    const uint16_t m = mk[k];
-    v[k] = 0;
-    if (m & kDomainBit) {
-      const int si = si0 + 100 * k;
-      const T ec = ecs[k];
-      T me = 0;
-#pragma unroll
-      for (int f = 0; f < 6; ++f) {
-        if (m & (1u << (8 + f))) me += ih2[f >> 1] * ec;
-        if (m & (1u << f)) me -= ih2[f >> 1] * zrun_nbr(se, ecs, si, k, f);
-      }
-      v[k] = (T)rk[k] - me;
-    }
-  }
-  // the 2x2x2 children of a level-1 cell: z pairs inside the thread's run,
-  // x pairs on lanes t, t ^ 1 and y pairs on lanes t, t ^ 8 (x = t & 7,
-  // y = (t >> 3) & 7); the lane with x and y even holds the sums
-  T s0 = v[0] + v[1], s1 = v[2] + v[3];
-  s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
-  s1 += __shfl_xor_sync(0xffffffffu, s1, 1);
-  s0 += __shfl_xor_sync(0xffffffffu, s0, 8);
-  s1 += __shfl_xor_sync(0xffffffffu, s1, 8);
-  const int x = threadIdx.x & 7, y = (threadIdx.x >> 3) & 7, zh = threadIdx.x >> 6;
-  if (!((x | y) & 1)) {
-    const size_t base = (size_t)b * 64 + (x >> 1) + 4 * (y >> 1) + 16 * (2 * zh);
-    r1[base] = s0;
-    r1[base + 16] = s1;
-  }
+  if (solve_done(done) || j >= nd) return;
+  T own[4][2];
+  HaloV<T> hv;
+  half_field<false>(s, h, e, e, own, hv);
+  half_restrict(s, h, mk, P, own, hv, rk, r1);
 }
 
 // Level-1 parent (within its brick's 64) of cell `off` of a level-0 brick.
 __device__ inline int parent_off(int off) { return ((off & 7) >> 1) + 4 * (((off >> 3) & 7) >> 1) + 16 * (off >> 7); }
 
 // Post-smoothing at level 0. FIRST: ep = e + P e1 (coarse correction added on
-// the fly, the level-1 parent of every staged cell read as it is staged), out
-// = ep + w D^-1 (r - M ep) into eout. Otherwise a plain sweep writing the FP64
-// preconditioned residual z and the block's partial r.z. The cells' r and
-// face masks are loaded first, so they are in flight during the staging.
+// the fly, the level-1 parent of every cell read with it), out = ep + w D^-1
+// (r - M ep). Otherwise a plain sweep that writes the preconditioned residual z
+// (in T, which the direction update widens: half the bytes in the FP32 form)
+// and the block's partial r.z. r was written many launches back.
 template <class T, bool FIRST>
-__global__ void __launch_bounds__(kBT, sizeof(T) == 4 ? 16 : 1) k0_post(const int* __restrict__ drow,
+__global__ void __launch_bounds__(kHT) k0_post(const int* __restrict__ drow, int nd,
                                                const uint16_t* __restrict__ fmask, const double* __restrict__ r,
-                                               const T* __restrict__ e, const T* __restrict__ e1, T* __restrict__ eout,
-                                               double* __restrict__ z, double* partial, Params P,
-                                               const int32_t* __restrict__ done) {
-  __shared__ int64_t sb[6];
-  __shared__ T se[kS1];  // e (plus the coarse correction when FIRST) with face halo
-  const T om = (T)(FIRST ? P.mgw1 : P.mgw2), ih2[3] = {(T)P.ih2[0], (T)P.ih2[1], (T)P.ih2[2]};
-  // prologue: brick, face neighbours, face masks (static), r and, when FIRST,
-  // the brick's pre-smoothed e (both written many launches back)
-  const int b = load_drow(drow, sb);
-  const int ob = zrun_base();  // the stencil pass's z-run (cells ob + 64 k)
-  uint16_t mk[kCPT];
-  double rk[kCPT];
+                                               const T* __restrict__ e, const T* __restrict__ e1, T* __restrict__ out,
+                                               double* partial, Params P, const int32_t* __restrict__ done) {
+  const int j = blockIdx.x * kHB + (threadIdx.x >> 6), h = (threadIdx.x >> 5) & 1;
+  Half s;
+  uint32_t mk[4];
+  double rk[4][2];
+  if (j < nd) {
+    half_load(drow + 8 * (size_t)j, h, s);
+    half_masks(fmask, s, mk);
 #pragma unroll
-  for (int k = 0; k < kCPT; ++k) {
-    const int64_t c = (int64_t)b * kCells + ob + 64 * k;
-    mk[k] = fmask[c];
-    rk[k] = r[c];
+    for (int k = 0; k < 4; ++k) ld2(r + s.c + 64 * k, rk[k]);
   }
-  T v[4];
-  if (FIRST) load4(e + (int64_t)b * kCells + 4 * threadIdx.x, v);
   pdl_entry();
   if (solve_done(done)) return;
-  if (FIRST) {
-    // the brick: cells 4t..4t+3 of one row share two level-1 parents
-    const int o4 = 4 * threadIdx.x;
-    const int p0 = parent_off(o4);
-    const T c0 = e1[(size_t)b * 64 + p0], c1 = e1[(size_t)b * 64 + p0 + 1];
-    __syncthreads();
-    stage_h1_halo(se, sb, [&](int64_t i) { return e[i] + e1[(i >> 9) * 64 + parent_off((int)(i & 511))]; });
-    const int si = s1_of(o4);
-    se[si] = v[0] + c0;
-    se[si + 1] = v[1] + c0;
-    se[si + 2] = v[2] + c1;
-    se[si + 3] = v[3] + c1;
-  } else {
-    __syncthreads();
-    stage_arr(se, e, b, sb);
-  }
-  __syncthreads();
-  const int si0 = s1_of(ob);
-  T eps[kCPT];
-#pragma unroll
-  for (int k = 0; k < kCPT; ++k) eps[k] = se[si0 + 100 * k];
   double rz = 0;
-#pragma unroll
-  for (int k = 0; k < kCPT; ++k) {
-    const int64_t c = (int64_t)b * kCells + ob + 64 * k;
-    const uint16_t m = mk[k];
-    if (!(m & kDomainBit)) {
-      if (FIRST) eout[c] = (T)0;
-      else z[c] = 0.0;
-      continue;
-    }
-    const int si = si0 + 100 * k;
-    const T epc = eps[k];
-    T me = 0;
-#pragma unroll
-    for (int f = 0; f < 6; ++f) {
-      if (m & (1u << (8 + f))) me += ih2[f >> 1] * epc;
-      if (m & (1u << f)) me -= ih2[f >> 1] * zrun_nbr(se, eps, si, k, f);
-    }
-    double rc = rk[k];
-    T out = epc + om * (T)P.dtab[active_index(m)] * ((T)rc - me);
-    if (FIRST) {
-      eout[c] = out;
-    } else {
-      z[c] = (double)out;
-      rz += rc * (double)out;
-    }
+  if (j < nd) {
+    T own[4][2];
+    HaloV<T> hv;
+    half_field<FIRST>(s, h, e, e1, own, hv);
+    rz = half_sweep(s, mk, [&](uint16_t m) { return (T)P.dtab[active_index(m)]; }, P, (T)(FIRST ? P.mgw1 : P.mgw2), own,
+                    hv, rk, out);
   }
-  if (!FIRST) block_sum<kBT>(rz, 0.0, partial);
+  if (!FIRST) block_sum<kHT>(rz, 0.0, partial);
 }
 
 // ---- level 0 with one sweep before and after the coarse correction.
@@ -1649,6 +1526,7 @@ static void mg_vcycle_t(Ctx* c, int update, int part) {
   const int32_t* dn = &c->ds->done;
   // down (with update: finish the previous CG iteration into r2, which becomes r)
   const bool one = c->mg_sweeps0 == 1;
+  const int gh = half_blocks(nd);
   if (part & 1) {
     c->npart_head = nd;
     if (c->mg_bulk && c->bulk_grid > 0) {
@@ -1665,7 +1543,8 @@ static void mg_vcycle_t(Ctx* c, int update, int part) {
       launch_k(c, k0_pre_restrict<T>, nd, kBT, 0, c->drow, c->fmask, c->r, c->r2, c->x, c->pd, c->q, c->partial,
                c->ds, update, r1, c->dp); MAC_COUNT(c);
     } else {
-      launch_k(c, k0_pre<T>, nd, kBT, 0, c->drow, c->fmask, c->r, c->r2, c->x, c->pd, c->q, c->partial, c->ds,
+      c->npart_head = gh;
+      launch_k(c, k0_pre<T>, gh, kHT, 0, c->drow, nd, c->fmask, c->r, c->r2, c->x, c->pd, c->q, c->partial, c->ds,
                update, e0, c->dp); MAC_COUNT(c);
     }
     if (update) {
@@ -1675,7 +1554,7 @@ static void mg_vcycle_t(Ctx* c, int update, int part) {
   }
   if (!(part & 2)) return;
   if (!one) {
-    launch_k(c, k0_restrict<T>, nd, kBT, 0, c->drow, c->fmask, c->r, e0, r1, c->dp, dn); MAC_COUNT(c);
+    launch_k(c, k0_restrict<T>, gh, kHT, 0, c->drow, nd, c->fmask, c->r, e0, r1, c->dp, dn); MAC_COUNT(c);
   }
   const T sw1 = (T)c->dp.mgw1, sw2 = (T)c->dp.mgw2;
   launch_k(c, kl_pre<T, 4>, g1, 256, 0, c->drow, nd, w1, ncap1, r1, e1, sw1, sw2, dn); MAC_COUNT(c);
@@ -1721,12 +1600,14 @@ static void mg_vcycle_t(Ctx* c, int update, int part) {
            sw2, dn); MAC_COUNT(c);
   if (one) {
     launch_k(c, k0_post_one<T>, nd, kBT, 0, c->drow, c->fmask, c->r, e1, c->z, c->partial, c->dp, dn); MAC_COUNT(c);
+    c->npart_tail = nd;
     return;
   }
-  launch_k(c, k0_post<T, true>, nd, kBT, 0, c->drow, c->fmask, c->r, e0, e1, e0b, nullptr, nullptr, c->dp,
+  launch_k(c, k0_post<T, true>, gh, kHT, 0, c->drow, nd, c->fmask, c->r, e0, e1, e0b, c->partial, c->dp,
            dn); MAC_COUNT(c);
-  launch_k(c, k0_post<T, false>, nd, kBT, 0, c->drow, c->fmask, c->r, e0b, nullptr, nullptr, c->z, c->partial,
-           c->dp, dn); MAC_COUNT(c);
+  launch_k(c, k0_post<T, false>, gh, kHT, 0, c->drow, nd, c->fmask, c->r, e0b, nullptr, (T*)c->z, c->partial, c->dp,
+           dn); MAC_COUNT(c);
+  c->npart_tail = gh;
 }
 
 void mg_vcycle(Ctx* c, int update, int part) {

@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "mac_internal.cuh"
+#include "mac_half.cuh"
 #include "mac_unet.cuh"
 
 namespace mac {
@@ -87,50 +88,44 @@ void free_solver(Ctx* c) {
 }
 
 // ------------------------------------------------------------ helpers
-// Sums the per-block partials in a fixed order (one block of 1024 threads).
-// Each thread first adds a strided run of partials with eight loads of each
-// array in flight (the partials sit in L2; a loop with one load per
-// iteration waited one L2 round trip per element).
-__device__ inline void sum_partials(const double* partial, int nblk, double* s0, double* s1) {
-  __shared__ double sa[32], sb[32];
-  double a = 0, b = 0;
+// Sums the per-block partials in a fixed order (one block of 1024 threads),
+// NS of the two runs of them. Each thread first adds a strided run of partials
+// with eight loads of each array in flight (the partials sit in L2; a loop with
+// one load per iteration waited one L2 round trip per element).
+template <int NS>
+__device__ inline void sum_partials(const double* partial, int nblk, double* out) {
+  __shared__ double sm[NS][32];
+  double a[NS] = {};
   const int step = blockDim.x;
   int i = threadIdx.x;
   for (; i + 7 * step < nblk; i += 8 * step) {
-    double va[8], vb[8];
+    double v[NS][8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      va[k] = __ldcg(partial + i + k * step);
-      vb[k] = __ldcg(partial + nblk + i + k * step);
-    }
+    for (int k = 0; k < 8; ++k)
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      a += va[k];
-      b += vb[k];
-    }
+      for (int n = 0; n < NS; ++n) v[n][k] = __ldcg(partial + n * nblk + i + k * step);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+#pragma unroll
+      for (int n = 0; n < NS; ++n) a[n] += v[n][k];
   }
-  for (; i < nblk; i += step) {
-    a += __ldcg(partial + i);
-    b += __ldcg(partial + nblk + i);
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    a += __shfl_down_sync(0xffffffffu, a, o);
-    b += __shfl_down_sync(0xffffffffu, b, o);
-  }
-  int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) {
-    sa[w] = a;
-    sb[w] = b;
+  for (; i < nblk; i += step)
+#pragma unroll
+    for (int n = 0; n < NS; ++n) a[n] += __ldcg(partial + n * nblk + i);
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+#pragma unroll
+  for (int n = 0; n < NS; ++n) {
+    for (int o = 16; o > 0; o >>= 1) a[n] += __shfl_down_sync(0xffffffffu, a[n], o);
+    if (l == 0) sm[n][w] = a[n];
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double ta = 0, tb = 0;
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) {
-      ta += sa[i];
-      tb += sb[i];
+  if (w == 0) {
+#pragma unroll
+    for (int n = 0; n < NS; ++n) {
+      double t = l < (int)(blockDim.x >> 5) ? sm[n][l] : 0.0;
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+      if (l == 0) out[n] = t;
     }
-    *s0 = ta;
-    *s1 = tb;
   }
 }
 
@@ -483,70 +478,40 @@ __global__ void __launch_bounds__(kBT) k_residual(const int* __restrict__ drow,
 
 // p = z + beta p (first: p = z), then q = M p and the partial p.q; the
 // neighbours' new p is formed on the fly so p is read once and written once.
-__global__ void __launch_bounds__(kBT) k_update_spmv(const int* __restrict__ drow,
-                                                     const uint16_t* __restrict__ fmask, const double* __restrict__ z,
+// Half bricks of one warp each, as the level-0 sweeps; Z is z's type (float
+// from the FP32 V-cycle's last sweep). z was written two launches back, p_old
+// in the last iteration; only beta comes from the previous launch.
+template <class Z>
+__global__ void __launch_bounds__(kHT) k_update_spmv(const int* __restrict__ drow, int nd,
+                                                     const uint16_t* __restrict__ fmask, const Z* __restrict__ z,
                                                      const double* __restrict__ pold, double* __restrict__ pnew,
                                                      double* __restrict__ q, double* partial, Params P,
                                                      const Scalars* ds, int first) {
-  __shared__ int64_t sb[6];
-  __shared__ double sp[kS1];  // the new direction on the brick and its face halo
-  // prologue: brick, face neighbours and face masks (static), the brick's z
-  // (the preconditioner's output, two launches back) and p_old (16-byte
-  // vector loads); only beta comes from the previous launch
-  const int b = load_drow(drow, sb);
-  const int ob = zrun_base();  // the stencil pass's z-run (cells ob + 64 k)
-  uint16_t mk[kCPT];
-#pragma unroll
-  for (int k = 0; k < kCPT; ++k) mk[k] = fmask[(int64_t)b * kCells + ob + 64 * k];
-  const int o4 = 4 * threadIdx.x;
-  double vz[4], vp[4] = {0.0, 0.0, 0.0, 0.0};
-  load4(z + (int64_t)b * kCells + o4, vz);
-  if (!first) load4(pold + (int64_t)b * kCells + o4, vp);
+  const int j = blockIdx.x * kHB + (threadIdx.x >> 6), h = (threadIdx.x >> 5) & 1;
+  Half s;
+  uint32_t mk[4];
+  if (j < nd) {
+    half_load(drow + 8 * (size_t)j, h, s);
+    half_masks(fmask, s, mk);
+  }
   pdl_entry();
   if (ds->done) return;
   const double be = first ? 0.0 : ds->beta;
-  __syncthreads();
-  // p = z (first) or z + beta p_old, on the brick and its face halo
-  if (first) stage_h1_halo(sp, sb, [&](int64_t i) { return z[i]; });
-  else stage_h1_halo(sp, sb, [&](int64_t i) { return z[i] + be * pold[i]; });
-  const int si4 = s1_of(o4);
-#pragma unroll
-  for (int k = 0; k < 4; ++k) sp[si4 + k] = first ? vz[k] : vz[k] + be * vp[k];
-  __syncthreads();
-  const int si0 = s1_of(ob);
-  double pcs[kCPT];
-#pragma unroll
-  for (int k = 0; k < kCPT; ++k) pcs[k] = sp[si0 + 100 * k];
   double pq = 0;
-#pragma unroll
-  for (int k = 0; k < kCPT; ++k) {
-    const int64_t c = (int64_t)b * kCells + ob + 64 * k;
-    const uint16_t m = mk[k];
-    if (!(m & kDomainBit)) {
-      pnew[c] = 0.0;
-      q[c] = 0.0;
-      continue;
-    }
-    const int si = si0 + 100 * k;
-    const double pc = pcs[k];
-    double s = 0;
-#pragma unroll
-    for (int f = 0; f < 6; ++f) {
-      if (m & (1u << (8 + f))) s += P.ih2[f >> 1] * pc;
-      if (m & (1u << f)) s -= P.ih2[f >> 1] * zrun_nbr(sp, pcs, si, k, f);
-    }
-    pnew[c] = pc;
-    q[c] = s;
-    pq += pc * s;
+  if (j < nd) {
+    double own[4][2];
+    HaloV<double> hv;
+    half_direction(s, z, pold, be, first, own, hv);
+    pq = half_spmv(s, mk, P, own, hv, pnew, q);
   }
-  block_sum<kBT>(pq, 0.0, partial);
+  block_sum<kHT>(pq, 0.0, partial);
 }
 
 __global__ void k_fin_alpha(const double* partial, int nblk, Scalars* ds) {
   pdl_entry();
   if (ds->done) return;
-  double pq, unused;
-  sum_partials(partial, nblk, &pq, &unused);
+  double pq = 0;
+  sum_partials<1>(partial, nblk, &pq);
   if (threadIdx.x == 0) {
     ds->pq = pq;
     ds->alpha = pq != 0 ? ds->rz / pq : 0.0;
@@ -570,8 +535,8 @@ __global__ void __launch_bounds__(512) k_axpy(const int* __restrict__ dbl, doubl
 __global__ void k_fin_rr(const double* partial, int nblk, Scalars* ds, double rtol2, int max_iters) {
   pdl_entry();
   if (ds->done) return;
-  double rr, unused;
-  sum_partials(partial, nblk, &rr, &unused);
+  double rr = 0;
+  sum_partials<1>(partial, nblk, &rr);
   if (threadIdx.x == 0) {
     ds->rr = rr;
     ds->iters += 1;
@@ -581,8 +546,8 @@ __global__ void k_fin_rr(const double* partial, int nblk, Scalars* ds, double rt
 
 __global__ void k_fin_bnorm(const double* partial, int nblk, Scalars* ds) {
   pdl_entry();
-  double bb, unused;
-  sum_partials(partial, nblk, &bb, &unused);
+  double bb = 0;
+  sum_partials<1>(partial, nblk, &bb);
   if (threadIdx.x == 0) {
     ds->bnorm2 = bb;
     ds->rr = bb;
@@ -593,8 +558,8 @@ __global__ void k_fin_bnorm(const double* partial, int nblk, Scalars* ds) {
 
 __global__ void k_fin_rr_initial(const double* partial, int nblk, Scalars* ds, double rtol2) {
   pdl_entry();
-  double rr, unused;
-  sum_partials(partial, nblk, &rr, &unused);
+  double rr = 0;
+  sum_partials<1>(partial, nblk, &rr);
   if (threadIdx.x == 0) {
     ds->rr = rr;
     if (rr <= rtol2 * ds->bnorm2) ds->done = 1;
@@ -605,8 +570,8 @@ __global__ void k_fin_rr_initial(const double* partial, int nblk, Scalars* ds, d
 __global__ void k_fin_beta(const double* partial, int nblk, Scalars* ds, int first) {
   pdl_entry();
   if (ds->done) return;
-  double rz, unused;
-  sum_partials(partial, nblk, &rz, &unused);
+  double rz = 0;
+  sum_partials<1>(partial, nblk, &rz);
   if (threadIdx.x == 0) {
     ds->beta = first ? 0.0 : (ds->rz != 0 ? rz / ds->rz : 0.0);
     ds->rz = rz;
@@ -794,9 +759,10 @@ __global__ void __launch_bounds__(512) k_from_dense(const int* __restrict__ dbl,
 // beta = (r.z - r.zold) / rz_prev (Polak-Ribiere; 0 on a restart), rz = r.z
 __global__ void k_fin_beta_flex(const double* partial, int nblk, Scalars* ds, int first) {
   if (ds->done) return;
-  double rz, rzo;
-  sum_partials(partial, nblk, &rz, &rzo);
+  double sums[2] = {};
+  sum_partials<2>(partial, nblk, sums);
   if (threadIdx.x == 0) {
+    const double rz = sums[0], rzo = sums[1];
     ds->beta = first ? 0.0 : (ds->rz != 0 ? (rz - rzo) / ds->rz : 0.0);
     ds->rz = rz;
   }
@@ -997,17 +963,24 @@ int project_field(Ctx* c, double* const* U, const double* const* D, int more) {
       prof_end(c, PH_VCYCLE);
       prof_begin(c, PH_CGVEC);
       if (!learned) {
-        launch_k(c, k_fin_beta, 1, 1024, 0, c->partial, nd, c->ds, first); MAC_COUNT(c);
+        launch_k(c, k_fin_beta, 1, 1024, 0, c->partial, fold ? c->npart_tail : nd, c->ds, first); MAC_COUNT(c);
       }
       prof_end(c, PH_CGVEC);
       prof_begin(c, PH_SPMV);
       std::swap(c->pd, c->pd2);  // pd2: previous direction, pd: new one
-      launch_k(c, k_update_spmv, nd, kBT, 0, c->drow, c->fmask, c->z, c->pd2, c->pd, c->q, c->partial, c->dp, c->ds,
-               first); MAC_COUNT(c);
+      // the two-sweep V-cycle leaves z in its own type
+      const int gh = half_blocks(nd);
+      if (fold && c->mg_float && c->mg_sweeps0 != 1) {
+        launch_k(c, k_update_spmv<float>, gh, kHT, 0, c->drow, nd, c->fmask, (const float*)c->z, c->pd2, c->pd, c->q,
+                 c->partial, c->dp, c->ds, first); MAC_COUNT(c);
+      } else {
+        launch_k(c, k_update_spmv<double>, gh, kHT, 0, c->drow, nd, c->fmask, c->z, c->pd2, c->pd, c->q, c->partial,
+                 c->dp, c->ds, first); MAC_COUNT(c);
+      }
       prof_end(c, PH_SPMV);
       first = 0;
       prof_begin(c, PH_CGVEC);
-      launch_k(c, k_fin_alpha, 1, 1024, 0, c->partial, nd, c->ds); MAC_COUNT(c);
+      launch_k(c, k_fin_alpha, 1, 1024, 0, c->partial, gh, c->ds); MAC_COUNT(c);
       if (!fold) {
         launch_k(c, k_axpy, nd, 512, 0, c->dbl, c->x, c->r, c->pd, c->q, c->partial, c->ds); MAC_COUNT(c);
         launch_k(c, k_fin_rr, 1, 1024, 0, c->partial, nd, c->ds, rtol2, c->prm.max_iters); MAC_COUNT(c);
