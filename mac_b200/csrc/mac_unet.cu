@@ -515,39 +515,53 @@ __global__ void __launch_bounds__(128) k_wgrad(WgradArgs a) {
 // --------------------------------- 3x3x3 convolutions marching along z
 // A CTA owns an 8 (x) x 16 (y) tile of voxels and walks it through a run of z
 // planes. The input planes of the tile with a one-voxel halo (10 x 18 voxels x
-// KC channels) pass through a ring of four in shared memory, in the no-swizzle
-// K-major layout [channel group][y][x] x 16 bytes: a tap's A operand is the
-// planes seen from another start address (M-adjacent core matrices 160 bytes
-// apart, K-adjacent ones a channel group). Each plane is gathered once a run
-// where a box per plane gathers three, the next plane's loads are in flight in
-// registers while the tensor core works on this one, the epilogue of the plane
-// before (bias, ReLU, BF16 store) runs meanwhile, and the weights of all taps
-// are staged once a run. Two accumulators alternate in tensor memory. The
-// accumulation visits taps and K steps in k_conv's order.
+// KC channels) pass one by one through two buffers in shared memory, in the
+// no-swizzle K-major layout [channel group][y][x] x 16 bytes: a tap's A operand
+// is the plane seen from another start address (M-adjacent core matrices 160
+// bytes apart, K-adjacent ones a channel group). An input plane belongs to the
+// sums of three output planes; their accumulators lie side by side in a ring in
+// tensor memory and the weights of the three dz side by side in B, so that one
+// MMA of 3 NC columns does the three (an MMA of 128 rows takes about 80 cycles up
+// to 48 columns: A's reading from shared memory bounds it). Where the window of
+// three crosses the ring's end, and for the first product of a new output plane
+// (which overwrites the accumulator), it is two MMAs. The next plane's loads are
+// in flight in registers while the tensor core works on this one, the epilogue
+// of the last finished plane (bias, ReLU, BF16 store) runs meanwhile, and the
+// weights of all taps are staged once a run. An output plane's sum visits taps
+// and K steps in k_conv's order: its first nine taps come with the first of its
+// three input planes.
 //
-// MODE 0 is the forward convolution, MODE 1 the input gradient (negated taps, B
-// MN-major), as in k_conv. What bounds it is the tensor core's
-// reading of A from shared memory: 27 KC/16 operands of 4 KB a plane. Measured
-// on one B200 (before: a box per output plane, or a gather per tap in MODE 1):
-// forward at 128^3, 16 -> 16 channels 166 -> 108 us, 32 -> 16 569 -> 320 us;
-// input gradient of 16 x 64^3, 16 -> 16 812 -> 231 us.
-constexpr int kPlX = 10, kPlY = 18, kPlVox = kPlX * kPlY, kRing = 4;
+// MODE 0 is the forward convolution (planes upwards), MODE 1 the input gradient
+// (negated taps, so planes downwards; B MN-major), as in k_conv. Measured on one
+// B200 (first a box per output plane or a gather per tap in MODE 1, then a march
+// with one dz an MMA, now), us: forward at 128^3, 16 -> 16 channels 166, 108, 83,
+// 32 -> 16 569, 320, 158; input gradient of 16 x 64^3, 16 -> 16 812, 231, 122.
+constexpr int kPlX = 10, kPlY = 18, kPlVox = kPlX * kPlY;
 
+// Shared memory, accumulators in the ring and CTAs an SM: eight accumulators
+// (the window of three crosses the end in two of eight planes) unless four let
+// more CTAs share the 512 columns of tensor memory (16 -> 16 at 128^3: six CTAs
+// 83 us, four with eight accumulators each 101 us).
 template <int KC, int NC>
-__host__ __device__ constexpr int march_smem() {
-  return kRing * KC * kPlVox * 2 + 27 * NC * KC * 2 + 128;
-}
+struct March {
+  static constexpr int need = 2 * KC * kPlVox * 2 + 27 * NC * KC * 2 + 128;
+  static constexpr int by_smem = 227 * 1024 / (need + 1024) < 6 ? 227 * 1024 / (need + 1024) : 6;  // 6: registers
+  static constexpr int ring = 512 / (8 * NC) >= by_smem ? 8 : 4;
+  static constexpr int by_tmem = 512 / (ring * NC);
+  static constexpr int occ = by_smem < by_tmem ? by_smem : by_tmem;
+  // no more CTAs may be resident than tensor memory has room for
+  static constexpr int least = 227 * 1024 / (by_tmem + 1) + 1;
+  static constexpr int smem = need > least ? need : least;
+};
 
 template <int KC, int NC, int MODE>
-__global__ void __launch_bounds__(128) k_conv_march(ConvArgs a, int zrun) {
+__global__ void __launch_bounds__(128, March<KC, NC>::occ) k_conv_march(ConvArgs a, int zrun) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  constexpr int G = KC / 8, PLANE = G * kPlVox * 16, CH = (G * kPlVox + 127) / 128;
+  constexpr int G = KC / 8, PLANE = G * kPlVox * 16, CH = (G * kPlVox + 127) / 128, R = March<KC, NC>::ring;
   constexpr int NB = CH > 6 ? 6 : CH;  // chunks of a plane held in registers at a time
-  constexpr uint32_t LBO_A = kPlVox * 16, SBO_A = kPlX * 16, SBO_B = (KC / 8) * 128;
-  constexpr uint32_t ACC = NC < 16 ? 16 : NC, TCOLS = 2 * ACC < 32 ? 32 : 2 * ACC;
-  constexpr uint32_t IDESC = umma::idesc_bf16(128, NC, 0, MODE);
-  uint8_t* wbuf = smem + kRing * PLANE;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(wbuf + 27 * NC * KC * 2);
+  constexpr uint32_t LBO_A = kPlVox * 16, SBO_A = kPlX * 16, SBO_B = (KC / 8) * 128, WT = NC * KC * 2;
+  uint8_t* wbuf = smem + 2 * PLANE;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(wbuf + 27 * WT);
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 2);
   const int tid = threadIdx.x, warp = tid >> 5;
   const int tx = (a.w + 7) / 8, ty = (a.h + 15) / 16;
@@ -563,38 +577,51 @@ __global__ void __launch_bounds__(128) k_conv_march(ConvArgs a, int zrun) {
     umma::mbar_init(&bars[1], 1);
     fence_barrier_init();
   }
-  if (warp == 0) umma::tmem_alloc(tslot, TCOLS);
-  // chunk i = tid + 128 q of a plane: channel group i / 180, voxel i % 180
-  auto fetch = [&](int z, int q) -> uint4 {
+  if (warp == 0) umma::tmem_alloc(tslot, R * NC);
+  // input plane i of the run feeds its output planes i - 2, i - 1 and i
+  const int nout = z1 - z0, nin = nout + 2;
+  auto zin = [&](int i) { return MODE ? z1 - i : z0 - 1 + i; };
+  // chunk q of a thread: cell tid + 128 q of the plane's [channel group][voxel]; its place in a plane of its source
+  // (16-byte units, lowest bit the source; -1 outside the grid) does not change along the run
+  int place[CH];
+#pragma unroll
+  for (int q = 0; q < CH; ++q) {
     const int i = tid + 128 * q, g = i / kPlVox, vox = i - g * kPlVox, by = vox / kPlX;
-    const int x = x0 - 1 + vox - by * kPlX, y = y0 - 1 + by;
-    uint4 v = make_uint4(0, 0, 0, 0);
-    if (i < G * kPlVox && z >= 0 && z < a.d && y >= 0 && y < a.h && x >= 0 && x < a.w)
-      v = gather8(a.s1, a.s2, g, n, z, y, x, a.d, a.h, a.w);
-    return v;
+    const int x = x0 - 1 + vox - by * kPlX, y = y0 - 1 + by, second = 8 * g >= a.s1.c;
+    const Src& s = second ? a.s2 : a.s1;
+    const int gg = second ? g - a.s1.c / 8 : g;
+    const bool in = i < G * kPlVox && y >= 0 && y < a.h && x >= 0 && x < a.w;
+    place[q] = in ? 2 * (((y >> s.shift) * (a.w >> s.shift) + (x >> s.shift)) * (s.c / 8) + gg) + second : -1;
+  }
+  auto plane = [&](const Src& s, int z) {
+    return s.p + ((size_t)n * (a.d >> s.shift) + (z >> s.shift)) * (a.h >> s.shift) * (a.w >> s.shift) * s.c;
   };
-  auto put = [&](int z, int q, uint4 v) {
+  auto fetch = [&](int z, int q) -> uint4 {
+    if (z < 0 || z >= a.d || place[q] < 0) return make_uint4(0, 0, 0, 0);
+    return ldg16((place[q] & 1 ? plane(a.s2, z) : plane(a.s1, z)) + (size_t)(place[q] >> 1) * 8);
+  };
+  auto put = [&](int buf, int q, uint4 v) {
     const int i = tid + 128 * q;
-    if (i < G * kPlVox) *reinterpret_cast<uint4*>(smem + ((z + kRing) % kRing) * PLANE + i * 16) = v;
+    if (i < G * kPlVox) *reinterpret_cast<uint4*>(smem + buf * PLANE + i * 16) = v;
   };
-  for (int z = z0 - 1; z <= z0 + 1; ++z)
 #pragma unroll
-    for (int q0 = 0; q0 < CH; q0 += NB) {
-      uint4 v[NB];
+  for (int q0 = 0; q0 < CH; q0 += NB) {
+    uint4 v[NB];
 #pragma unroll
-      for (int q = 0; q < NB; ++q) v[q] = q0 + q < CH ? fetch(z, q0 + q) : make_uint4(0, 0, 0, 0);
+    for (int q = 0; q < NB; ++q) v[q] = q0 + q < CH ? fetch(zin(0), q0 + q) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-      for (int q = 0; q < NB; ++q)
-        if (q0 + q < CH) put(z, q0 + q, v[q]);
-    }
-  // weights of all taps: forward rows are output channels (K-major), input-gradient rows are K (MN-major)
+    for (int q = 0; q < NB; ++q)
+      if (q0 + q < CH) put(0, q0 + q, v[q]);
+  }
+  // weights of all taps, for each in-plane tap those of the last, middle and first third of the taps side by
+  // side; forward rows are output channels (K-major), input-gradient rows are K (MN-major)
   constexpr int ROWS = MODE ? KC : NC, WCH = MODE ? NC / 8 : KC / 8;
   for (int i = tid; i < 27 * ROWS * WCH; i += 128) {
     const int t = i / (ROWS * WCH), rem = i - t * ROWS * WCH, row = rem / WCH, c = rem % WCH;
     const uint4 v = ldg16(a.wt + (size_t)t * NC * KC + (size_t)row * WCH * 8 + c * 8);
     const uint32_t off = MODE ? (c * SBO_B + (row >> 3) * 128 + (row & 7) * 16)
                               : ((row >> 3) * SBO_B + c * 128 + (row & 7) * 16);
-    *reinterpret_cast<uint4*>(wbuf + (size_t)t * NC * KC * 2 + off) = v;
+    *reinterpret_cast<uint4*>(wbuf + (size_t)((t % 9) * 3 + 2 - t / 9) * WT + off) = v;
   }
   umma::fence_before_sync();
   __syncthreads();
@@ -602,9 +629,10 @@ __global__ void __launch_bounds__(128) k_conv_march(ConvArgs a, int zrun) {
   const uint32_t tmem = *tslot;
   const int mx = x0 + (tid & 7), my = y0 + (tid >> 3);  // TMEM lane = tile row: x = lane & 7, y = lane >> 3
   const bool valid = mx < a.w && my < a.h;
-  auto epilogue = [&](int z) {
+  auto epilogue = [&](int o) {
+    const int z = MODE ? z1 - 1 - o : z0 + o;
     const size_t v = (((size_t)n * a.d + z) * a.h + my) * a.w + mx;
-    const uint32_t trow = tmem + ((z - z0) & 1) * ACC + ((uint32_t)(warp * 32) << 16);
+    const uint32_t trow = tmem + (o % R) * NC + ((uint32_t)(warp * 32) << 16);
 #pragma unroll
     for (int c0 = 0; c0 < NC; c0 += 16) {
       float f[16];
@@ -634,65 +662,75 @@ __global__ void __launch_bounds__(128) k_conv_march(ConvArgs a, int zrun) {
     }
   };
   bool ok = true;
-  for (int z = z0; z < z1; ++z) {
+  for (int i = 0; i < nin; ++i) {
     umma::fence_before_sync();  // the epilogue's reads of the accumulator this plane overwrites
     umma::fence_async_smem();
     ok = __syncthreads_and(ok);
     if (!ok) break;
-    const int k = z - z0;
     if (tid == 0) {
       umma::fence_after_sync();
-      const uint32_t b0 = umma::smem_addr(wbuf), acc = tmem + (k & 1) * ACC;
-      for (int t = 0; t < 27; ++t) {
-        int dz, dy, dx;
-        tap_offset(t, 27, dz, dy, dx);
-        if (MODE == 1) {
-          dz = -dz;
-          dy = -dy;
-          dx = -dx;
-        }
-        const uint32_t at = umma::smem_addr(smem) + ((z + dz + kRing) % kRing) * PLANE + ((1 + dy) * kPlX + 1 + dx) * 16;
-        const uint32_t bt = b0 + t * NC * KC * 2;
+      const uint32_t b0 = umma::smem_addr(wbuf), p0 = umma::smem_addr(smem) + (i & 1) * PLANE;
+      const int lo = max(i - 2, 0), hi = min(i, nout - 1);
+#pragma unroll 1
+      for (int r = 0; r < 9; ++r) {
+        const int dy = MODE ? 1 - r / 3 : r / 3 - 1, dx = MODE ? 1 - r % 3 : r % 3 - 1;
+        const uint32_t at = p0 + (uint32_t)(((1 + dy) * kPlX + 1 + dx) * 16);
+        const uint32_t bt = b0 + 3 * r * WT;
 #pragma unroll
-        for (int ks = 0; ks < KC / 16; ++ks)
-          umma::mma(acc, umma::desc(at + ks * 2 * LBO_A, LBO_A, SBO_A), umma::desc(bt + ks * 256, 128, SBO_B), IDESC,
-                    (t > 0 || ks > 0) ? 1u : 0u);
+        for (int ks = 0; ks < KC / 16; ++ks) {
+          const uint64_t ad = umma::desc(at + ks * 2 * LBO_A, LBO_A, SBO_A);
+          // output planes o0 .. o1, contiguous in the ring
+          auto part = [&](int o0, int o1, uint32_t add) {
+            umma::mma(tmem + (o0 % R) * NC, ad, umma::desc(bt + (uint32_t)(o0 - i + 2) * WT + ks * 256, 128, SBO_B),
+                      umma::idesc_bf16(128, (o1 - o0 + 1) * NC, 0, MODE), add);
+          };
+          auto window = [&](int o0, int o1) {
+            const int e = o0 - o0 % R + R - 1;  // the last output plane before the ring's end
+            part(o0, min(o1, e), 1u);
+            if (o1 > e) part(e + 1, o1, 1u);
+          };
+          if (r == 0 && ks == 0 && hi == i) {
+            if (lo < i) window(lo, i - 1);
+            part(i, i, 0u);
+          } else {
+            window(lo, hi);
+          }
+        }
       }
-      umma::commit(&bars[k & 1]);
+      umma::commit(&bars[i & 1]);
     }
-    // plane z + 2 replaces plane z - 2, which the MMAs of plane z - 1 were the last to read
-    const bool more = z + 1 < z1;
+    // plane i + 1 replaces plane i - 1, which the MMAs of the iteration before read
+    const bool more = i + 1 < nin;
     uint4 v[NB];
     if (more) {
 #pragma unroll
-      for (int q = 0; q < NB; ++q) v[q] = fetch(z + 2, q);
+      for (int q = 0; q < NB; ++q) v[q] = fetch(zin(i + 1), q);
     }
-    if (k > 0) {
-      ok = umma::mbar_wait(&bars[(k - 1) & 1], ((k - 1) >> 1) & 1);
+    if (i > 0) {
+      ok = umma::mbar_wait(&bars[(i - 1) & 1], ((i - 1) >> 1) & 1);
       umma::fence_after_sync();
     }
     if (more) {
 #pragma unroll
-      for (int q = 0; q < NB; ++q) put(z + 2, q, v[q]);
+      for (int q = 0; q < NB; ++q) put((i + 1) & 1, q, v[q]);
 #pragma unroll
       for (int q0 = NB; q0 < CH; q0 += NB) {
 #pragma unroll
-        for (int q = 0; q < NB; ++q) v[q] = q0 + q < CH ? fetch(z + 2, q0 + q) : make_uint4(0, 0, 0, 0);
+        for (int q = 0; q < NB; ++q) v[q] = q0 + q < CH ? fetch(zin(i + 1), q0 + q) : make_uint4(0, 0, 0, 0);
 #pragma unroll
         for (int q = 0; q < NB; ++q)
-          if (q0 + q < CH) put(z + 2, q0 + q, v[q]);
+          if (q0 + q < CH) put((i + 1) & 1, q0 + q, v[q]);
       }
     }
-    if (k > 0 && __all_sync(0xffffffffu, ok)) epilogue(z - 1);
+    if (i > 2 && __all_sync(0xffffffffu, ok)) epilogue(i - 3);  // finished by plane i - 1
   }
-  const int last = z1 - 1 - z0;
-  if (ok) ok = umma::mbar_wait(&bars[last & 1], (last >> 1) & 1);
+  if (ok) ok = umma::mbar_wait(&bars[(nin - 1) & 1], ((nin - 1) >> 1) & 1);
   umma::fence_after_sync();
-  if (__syncthreads_and(ok)) epilogue(z1 - 1);
+  if (__syncthreads_and(ok)) epilogue(nout - 1);
   else if (tid == 0) atomicExch(a.err, 1);
   umma::fence_before_sync();
   __syncthreads();
-  if (warp == 0) umma::tmem_dealloc(tmem, TCOLS);
+  if (warp == 0) umma::tmem_dealloc(tmem, R * NC);
 }
 
 // --------------------------------------- 3x3x3 weight gradient from staged lines
@@ -1325,12 +1363,11 @@ static int march_run(const long tiles, int d, int want) {
 
 template <int KC, int NC, int MODE>
 static void conv_march_t(const ConvArgs& a, cudaStream_t st) {
-  constexpr int smem = march_smem<KC, NC>();
-  cudaFuncSetAttribute(k_conv_march<KC, NC, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  using M = March<KC, NC>;
+  cudaFuncSetAttribute(k_conv_march<KC, NC, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, M::smem);
   const long tiles = (long)a.n * ((a.h + 15) / 16) * ((a.w + 7) / 8);
-  constexpr int occ = 220 * 1024 / (smem + 1024) < 8 ? 220 * 1024 / (smem + 1024) : 8;
-  const int zrun = march_run(tiles, a.d, 148 * occ);
-  k_conv_march<KC, NC, MODE><<<(unsigned)(tiles * ((a.d + zrun - 1) / zrun)), 128, smem, st>>>(a, zrun);
+  const int zrun = march_run(tiles, a.d, 148 * M::occ);
+  k_conv_march<KC, NC, MODE><<<(unsigned)(tiles * ((a.d + zrun - 1) / zrun)), 128, M::smem, st>>>(a, zrun);
 }
 
 // 3x3x3 convolutions: marching along z where all taps' weights fit beside the
