@@ -20,6 +20,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "mac_internal.cuh"
@@ -1480,7 +1482,134 @@ struct Net {
   int loss_cap = 0;
   long launches = 0;
   int staged_conv = 1;  // 3x3x3 layers from staged planes (0: every tap gathered: k_conv, k_wgrad)
+  uint8_t* pinned = nullptr;  // staging of pageable host arrays: kCopyLanes x 2 slots, made on first use
+  cudaEvent_t slot_done[8] = {};
 };
+
+// ------------------------------------------------------------- host arrays
+// A caller's arrays are usually pageable, and the driver moves those through its
+// own buffer on the calling thread: 13-17 GB/s in, and out at the rate that one
+// thread faults fresh pages in. Above kCopyMin bytes the arrays go in chunks
+// through a small pinned buffer of the network instead, by a few lanes (threads)
+// that copy a chunk in or out while the link moves others. Registered or device
+// memory, small arrays and a failed staging allocation take the plain copy.
+// Measured on one B200 (16 cores): forward at 128^3 (10.5 MB in, 8.4 MB out) 3.15
+// -> 2.25 ms, loss and gradient of 16 x 64^3 (38 MB in) 11.0 -> 9.3 ms.
+constexpr int kCopyLanes = 4;
+constexpr size_t kCopyChunk = 512 * 1024, kCopyMin = 2 * 1024 * 1024;
+struct HostCopy {
+  void* dev;
+  void* host;
+  size_t bytes;
+};
+
+static bool copy_staging(Net& t) {
+  if (t.pinned) return true;
+  uint8_t* p = nullptr;
+  if (cudaMallocHost((void**)&p, 2 * kCopyLanes * kCopyChunk) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  for (int i = 0; i < 2 * kCopyLanes; ++i)
+    if (!t.slot_done[i] && cudaEventCreateWithFlags(&t.slot_done[i], cudaEventDisableTiming) != cudaSuccess) {
+      cudaGetLastError();
+      cudaFreeHost(p);
+      return false;
+    }
+  t.pinned = p;
+  return true;
+}
+
+// Lane l's chunks l, l + kCopyLanes, ... of the list, two slots alternating; the
+// copies go to the legacy default stream, as the network's kernels do.
+static int copy_lane(Net& t, const HostCopy* list, int n, bool up, int l) {
+  int rc = cuda_ok(cudaSetDevice(t.device));
+  struct Chunk {
+    uint8_t *dev, *host;
+    size_t bytes;
+  };
+  int i = 0;
+  size_t off = 0, index = 0;  // the list's next chunk
+  auto next = [&](Chunk* c) {
+    for (;; ++index, off += kCopyChunk) {
+      while (i < n && off >= list[i].bytes) {
+        ++i;
+        off = 0;
+      }
+      if (i == n) return false;
+      if (index % kCopyLanes == (size_t)l) break;
+    }
+    *c = Chunk{(uint8_t*)list[i].dev + off, (uint8_t*)list[i].host + off, std::min(kCopyChunk, list[i].bytes - off)};
+    ++index;
+    off += kCopyChunk;
+    return true;
+  };
+  Chunk c[2];
+  bool have[2] = {false, false};
+  // up: fill a slot when its last copy is done and send it; down: receive a chunk
+  // into a slot, and write out the one before meanwhile
+  for (int k = 0; !rc; k ^= 1) {
+    uint8_t* slot = t.pinned + (size_t)(2 * l + k) * kCopyChunk;
+    cudaEvent_t ev = t.slot_done[2 * l + k];
+    have[k] = next(&c[k]);
+    if (have[k]) {
+      if (up) {
+        rc = cuda_ok(cudaEventSynchronize(ev));
+        if (!rc) {
+          std::memcpy(slot, c[k].host, c[k].bytes);
+          rc = cuda_ok(cudaMemcpyAsync(c[k].dev, slot, c[k].bytes, cudaMemcpyHostToDevice, 0));
+        }
+      } else {
+        rc = cuda_ok(cudaEventSynchronize(ev));
+        if (!rc) rc = cuda_ok(cudaMemcpyAsync(slot, c[k].dev, c[k].bytes, cudaMemcpyDeviceToHost, 0));
+      }
+      if (!rc) rc = cuda_ok(cudaEventRecord(ev, 0));
+    }
+    if (!up && !rc && have[k ^ 1]) {
+      rc = cuda_ok(cudaEventSynchronize(t.slot_done[2 * l + (k ^ 1)]));
+      if (!rc) std::memcpy(c[k ^ 1].host, t.pinned + (size_t)(2 * l + (k ^ 1)) * kCopyChunk, c[k ^ 1].bytes);
+    }
+    if (!have[k]) break;
+  }
+  return rc;
+}
+
+// Copies the list in or out; a host array may be reused when it returns.
+static int copy_host(Net& t, const HostCopy* list, int n, bool up) {
+  size_t bytes = 0;
+  bool pageable = true;
+  for (int i = 0; i < n; ++i) {
+    cudaPointerAttributes at;
+    bytes += list[i].bytes;
+    if (cudaPointerGetAttributes(&at, list[i].host) != cudaSuccess) {
+      cudaGetLastError();
+      pageable = false;
+    } else if (at.type != cudaMemoryTypeUnregistered) {
+      pageable = false;
+    }
+  }
+  if (!pageable || bytes < kCopyMin || !copy_staging(t)) {
+    int rc = MAC_OK;
+    for (int i = 0; i < n && !rc; ++i)
+      rc = cuda_ok(up ? cudaMemcpy(list[i].dev, list[i].host, list[i].bytes, cudaMemcpyHostToDevice)
+                      : cudaMemcpy(list[i].host, list[i].dev, list[i].bytes, cudaMemcpyDeviceToHost));
+    return rc;
+  }
+  int rcs[kCopyLanes] = {};
+  std::thread lanes[kCopyLanes - 1];
+  int made = 0;
+  try {
+    for (; made < kCopyLanes - 1; ++made)
+      lanes[made] = std::thread([&, l = made + 1] { rcs[l] = copy_lane(t, list, n, up, l); });
+  } catch (const std::system_error&) {  // no thread to be had: this one does the rest
+  }
+  rcs[0] = copy_lane(t, list, n, up, 0);
+  for (int l = made + 1; l < kCopyLanes; ++l) rcs[l] = copy_lane(t, list, n, up, l);
+  for (int i = 0; i < made; ++i) lanes[i].join();
+  for (int l = 0; l < kCopyLanes; ++l)
+    if (rcs[l]) return rcs[l];
+  return MAC_OK;
+}
 
 static size_t level_vox(const Net& t, int l) {
   return (size_t)t.n * (t.d >> l) * (t.h >> l) * (t.w >> l);
@@ -1783,6 +1912,9 @@ void destroy(Net* t) {
   if (!t) return;
   cudaSetDevice(t->device);
   free_shape(*t);
+  if (t->pinned) cudaFreeHost(t->pinned);
+  for (cudaEvent_t ev : t->slot_done)
+    if (ev) cudaEventDestroy(ev);
   cudaFree(t->p);
   cudaFree(t->g);
   cudaFree(t->mo);
@@ -2051,11 +2183,11 @@ int mac_unet_forward(void* net, int n, int d, int h, int w, const float* r, cons
   int rc = mac::unet::ensure_shape(*t, n, d, h, w);
   if (rc) return rc;
   const size_t v0 = (size_t)n * d * h * w;
-  cudaMemcpy(t->r, r, v0 * 4, cudaMemcpyHostToDevice);
-  cudaMemcpy(t->m, mask, v0, cudaMemcpyHostToDevice);
-  rc = mac::unet::apply(t, 0);
+  const mac::unet::HostCopy in[2] = {{t->r, (void*)r, v0 * 4}, {t->m, (void*)mask, v0}}, res = {t->e, out, v0 * 4};
+  rc = mac::unet::copy_host(*t, in, 2, true);
+  if (!rc) rc = mac::unet::apply(t, 0);
   if (!rc) rc = mac::unet::check_err(*t, 0);
-  if (!rc) rc = mac::unet::cuda_ok(cudaMemcpy(out, t->e, v0 * 4, cudaMemcpyDeviceToHost));
+  if (!rc) rc = mac::unet::copy_host(*t, &res, 1, false);
   return rc;
 }
 
@@ -2067,10 +2199,9 @@ int mac_unet_loss_grad(void* net, int n, int d, int h, int w, const float* r, co
   int rc = mac::unet::ensure_shape(*t, n, d, h, w);
   if (rc) return rc;
   const size_t v0 = (size_t)n * d * h * w;
-  cudaMemcpy(t->r, r, v0 * 4, cudaMemcpyHostToDevice);
-  cudaMemcpy(t->m, mask, v0, cudaMemcpyHostToDevice);
-  cudaMemcpy(t->e, e, v0 * 4, cudaMemcpyHostToDevice);
-  rc = mac::unet::loss_grad(*t, t->loss, 0);
+  const mac::unet::HostCopy in[3] = {{t->r, (void*)r, v0 * 4}, {t->m, (void*)mask, v0}, {t->e, (void*)e, v0 * 4}};
+  rc = mac::unet::copy_host(*t, in, 3, true);
+  if (!rc) rc = mac::unet::loss_grad(*t, t->loss, 0);
   if (!rc) rc = mac::unet::check_err(*t, 0);
   if (!rc && loss) rc = mac::unet::cuda_ok(cudaMemcpy(loss, t->loss, sizeof(double), cudaMemcpyDeviceToHost));
   if (!rc && grad) rc = mac::unet::cuda_ok(cudaMemcpy(grad, t->g, t->np * 4, cudaMemcpyDeviceToHost));

@@ -63,7 +63,7 @@ class UNet:
         r = _f32(r)
         m = np.ascontiguousarray(mask, dtype=np.int8)
         n, d, h, w = r.shape
-        out = np.zeros_like(r)
+        out = np.empty_like(r)
         self._check(self.lib.mac_unet_forward(self.h, n, d, h, w, r.ctypes.data_as(_P(ctypes.c_float)),
                                               m.ctypes.data_as(_P(ctypes.c_int8)),
                                               out.ctypes.data_as(_P(ctypes.c_float))), "mac_unet_forward")
