@@ -297,80 +297,90 @@ __global__ void __launch_bounds__(256) k_layer_mask(const int* __restrict__ blis
 }
 
 // A face of a cell in brick b is written at level L only when its cell or the
-// cell behind it (-e_i) has layer L, so only when b or one of its -x, -y, -z
-// face neighbours holds a layer-L cell; other bricks are skipped whole.
-__global__ void __launch_bounds__(256) k_extrapolate(const int* __restrict__ blist, int nlive, const int* __restrict__ nbr,
+// cell behind it (-e_i) has layer L, so only when b or its -e_i face neighbour
+// holds a layer-L cell; other bricks are skipped whole.
+// A launch is a chain of dependent load rounds, not bandwidth, until the bricks
+// fill the device: SPLIT gives each axis a block of its own (blockIdx.y) with a
+// thread per cell, so a thread goes through one face's rounds instead of six;
+// otherwise a block takes the three axes, which share the cell's layers.
+template <bool SPLIT>
+__global__ void __launch_bounds__(SPLIT ? 512 : 256) k_extrapolate(const int* __restrict__ blist, int nlive,
+                                                     const int* __restrict__ nbr,
                                                      const int8_t* __restrict__ lay, const uint8_t* __restrict__ flags,
                                                      const uint32_t* __restrict__ lmask, double* fx, double* fy,
                                                      double* fz, int L) {
   pdl_entry();
-  double* const F[3] = {fx, fy, fz};
   __shared__ int sn[kNbr];
-  for (int bi = blockIdx.x; bi < nlive; bi += gridDim.x) {
-    int b = blist[bi];
-    if (threadIdx.x < kNbr) sn[threadIdx.x] = nbr[(size_t)b * kNbr + threadIdx.x];
-    __syncthreads();
-    uint32_t near = lmask[b];
+  const int b = blist[blockIdx.x];
+  if (threadIdx.x < kNbr) sn[threadIdx.x] = nbr[(size_t)b * kNbr + threadIdx.x];
+  const int i0 = SPLIT ? blockIdx.y : 0, i1 = SPLIT ? i0 + 1 : 3;
+  const uint32_t own = lmask[b];
+  __syncthreads();
+  uint32_t near = own;
+  for (int i = i0; i < i1; ++i) {
+    const int nb = sn[nbr_index(i == 0 ? -1 : 0, i == 1 ? -1 : 0, i == 2 ? -1 : 0)];
+    if (nb >= 0) near |= lmask[nb];
+  }
+  if (!(near & layer_bit(L))) return;
+  for (int o = threadIdx.x; o < kCells; o += blockDim.x) {
+    int64_t c = (int64_t)b * kCells + o;
+    int8_t lB = lay[c];
+    const uint8_t fl = flags[c];
+    int x = o & 7, y = (o >> 3) & 7, z = o >> 6;
+    // the layers behind the faces, in one round with the cell's own
+    int8_t la[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      if (!SPLIT || i == i0) la[i] = lay_i(lay, cidx(sn, x - (i == 0), y - (i == 1), z - (i == 2)));
+    if (lB < 0) continue;  // c must exist with a layer
+#pragma unroll
     for (int i = 0; i < 3; ++i) {
-      const int nb = sn[nbr_index(i == 0 ? -1 : 0, i == 1 ? -1 : 0, i == 2 ? -1 : 0)];
-      if (nb >= 0) near |= lmask[nb];
-    }
-    const bool skip = !(near & layer_bit(L));
-    for (int o = skip ? kCells : threadIdx.x; o < kCells; o += blockDim.x) {
-      int64_t c = (int64_t)b * kCells + o;
-      int8_t lB = lay[c];
-      if (lB < 0) continue;  // c must exist with a layer
-      int x = o & 7, y = (o >> 3) & 7, z = o >> 6;
-      uint8_t fl = flags[c];
-      // the layers behind the three faces, in one round
-      int8_t la[3];
+      if (SPLIT && i != i0) continue;
+      if (fl & (1u << i)) continue;  // non-forced Set on a const face does nothing
+      const int8_t lA = la[i];
+      const bool vA = lA >= 0;
+      const bool write = (vA && lA == L && lB >= L) || (lB == L && (!vA || lA >= L));
+      if (!write) continue;
+      double* Ui = i == 0 ? fx : (i == 1 ? fy : fz);
+      // Term k of the reference's sum, axis j = k / 2, sign s: a face whose
+      // layers and speed are loaded with all others before any is tested (a
+      // face waited on up to six dependent rounds, most of a small level's
+      // time: a 32 x 32 x 64 jet's step 1.05 -> 1.03 ms, a force-projection
+      // step of 45 levels 5% less, 29,000 bricks unchanged). j == i, s < 0: the
+      // face behind A, valid when A is; its own test layer is that of c - 2 e_i.
+      int64_t at[6];
+      int8_t l0[6], l1[6];
+      double v[6];
 #pragma unroll
-      for (int i = 0; i < 3; ++i) la[i] = lay_i(lay, cidx(sn, x - (i == 0), y - (i == 1), z - (i == 2)));
-#pragma unroll
-      for (int i = 0; i < 3; ++i) {
-        if (fl & (1u << i)) continue;  // non-forced Set on a const face does nothing
-        const int8_t lA = la[i];
-        const bool vA = lA >= 0;
-        const bool write = (vA && lA == L && lB >= L) || (lB == L && (!vA || lA >= L));
-        if (!write) continue;
-        const double* Ui = F[i];
-        // Term k of the reference's sum, axis j = k / 2, sign s: a face whose
-        // layers and speed are loaded with all others before any is tested (a
-        // face waited on up to six dependent rounds, most of a small level's
-        // time: a 32 x 32 x 64 jet's step 1.05 -> 1.03 ms, a force-projection
-        // step of 45 levels 5% less, 29,000 bricks unchanged). j == i, s < 0: the
-        // face behind A, valid when A is; its own test
-        // layer is that of c - 2 e_i.
-        int64_t at[6];
-        int8_t l0[6], l1[6];
-        double v[6];
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-          const int j = k >> 1, sg = (k & 1) ? 1 : -1;
-          const int mx = x + (j == 0 ? sg : 0), my = y + (j == 1 ? sg : 0), mz = z + (j == 2 ? sg : 0);
-          at[k] = cidx(sn, mx, my, mz);
-          l1[k] = lay_i(lay, at[k]);
-          if (j == i) l0[k] = sg < 0 ? lay_i(lay, cidx(sn, x - 2 * (i == 0), y - 2 * (i == 1), z - 2 * (i == 2))) : l1[k];
-          else l0[k] = lay_i(lay, cidx(sn, mx - (i == 0), my - (i == 1), mz - (i == 2)));
-          v[k] = rdv(Ui, at[k]);
-        }
-        int n = 0;
-        double val = 0;
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-          const bool take = (k >> 1) == i ? ((k & 1) || vA) && l0[k] >= 0 && l0[k] < L
-                                          : l0[k] >= 0 && l1[k] >= 0 && (l0[k] < L || l1[k] < L);
-          if (take) {
-            ++n;
-            val += v[k];
-          }
-        }
-        F[i][c] = val / n;
+      for (int k = 0; k < 6; ++k) {
+        const int j = k >> 1, sg = (k & 1) ? 1 : -1;
+        const int mx = x + (j == 0 ? sg : 0), my = y + (j == 1 ? sg : 0), mz = z + (j == 2 ? sg : 0);
+        at[k] = cidx(sn, mx, my, mz);
+        l1[k] = lay_i(lay, at[k]);
+        if (j == i) l0[k] = sg < 0 ? lay_i(lay, cidx(sn, x - 2 * (i == 0), y - 2 * (i == 1), z - 2 * (i == 2))) : l1[k];
+        else l0[k] = lay_i(lay, cidx(sn, mx - (i == 0), my - (i == 1), mz - (i == 2)));
+        v[k] = rdv(Ui, at[k]);
       }
+      int n = 0;
+      double val = 0;
+#pragma unroll
+      for (int k = 0; k < 6; ++k) {
+        const bool take = (k >> 1) == i ? ((k & 1) || vA) && l0[k] >= 0 && l0[k] < L
+                                        : l0[k] >= 0 && l1[k] >= 0 && (l0[k] < L || l1[k] < L);
+        if (take) {
+          ++n;
+          val += v[k];
+        }
+      }
+      Ui[c] = val / n;
     }
-    __syncthreads();
   }
 }
+
+// Live bricks up to which the three axes get blocks of their own (us a launch, one
+// block and three): 290 bricks 17.0 and 8.9, 588 bricks 22.0 and 13.4, 2,193 bricks
+// 26.8 and 30.7 (a block of three axes shares the loads of the layers).
+constexpr int kExtrapolateSplit = 1024;
 
 // Algorithms_Extrapolate on the vector field F (speed buffer 0 in pipeline A;
 // the stage speed and, through Algorithms_Accel_To_Speed, the acceleration in
@@ -379,9 +389,14 @@ int extrapolate_field(Ctx* c, double* const* F) {
   if (c->nlive_host == 0) return MAC_OK;
   prof_begin(c, PH_EXTRAPOLATE);
   launch_k(c, k_layer_mask, c->nlive_host, 256, 0, c->blist, c->lay, c->lmask); MAC_COUNT(c);
+  const int n = c->nlive_host;
   for (int L = 1; L <= c->dp.layer_max + 1; ++L) {
-    launch_k(c, k_extrapolate, c->nlive_host, 256, 0, c->blist, c->nlive_host, c->nbr, c->lay, c->flags, c->lmask,
-                                                        F[0], F[1], F[2], L); MAC_COUNT(c);
+    if (n <= kExtrapolateSplit)
+      launch_k(c, k_extrapolate<true>, dim3(n, 3), 512, 0, c->blist, n, c->nbr, c->lay, c->flags, c->lmask, F[0], F[1],
+               F[2], L);
+    else
+      launch_k(c, k_extrapolate<false>, n, 256, 0, c->blist, n, c->nbr, c->lay, c->flags, c->lmask, F[0], F[1], F[2], L);
+    MAC_COUNT(c);
   }
   prof_end(c, PH_EXTRAPOLATE);
   return check(cudaGetLastError());
