@@ -199,12 +199,13 @@ def roofline_models(ctx_stats, prof, np_count, n_exist, mg_bytes=8, cg_iteration
     # With one sweep on the finest level its pre- and post-sweep count once each:
     # (2 x 17 + 49) B there, the coarser levels (1/7 of 117 B) unchanged.
     vc = ((4.0 * 17.0 + 49.0) * 8.0 / 7.0 if sweeps0 == 2 else 2.0 * 17.0 + 49.0 + 117.0 / 7.0) * (mg_bytes / 8.0)
+    zb = mg_bytes if sweeps0 == 2 else 8  # the two-sweep V-cycle leaves z in its own type
     models = {
         # phase: (bytes per launch, description, launches or None for the region count)
         "move": (48.0 * np_count, "48 B per particle (read + write 3 FP64 positions)", None),
         "vcycle": ((vc + 48.0) * unk, f"{vc + 48.0:.1f} B per unknown per CG iteration: a V-cycle ({vc:.1f} B, "
                    f"levels 0.. at {mg_bytes} B per value) and the update it applies (48 B)", cg_iterations),
-        "spmv": (34.0 * unk, "34 B per unknown (read z, p_old 16, face mask 2, write p, q 16)", None),
+        "spmv": ((26.0 + zb) * unk, f"{26 + zb} B per unknown (read z {zb}, p_old 8, face mask 2, write p, q 16)", None),
         "forces": (75.0 * n_exist, "75 B per existing cell (mean of stage 1: 51, stage 2: 99)", None),
         "gradient": (67.0 * n_exist, "67 B per existing cell (x 8, flags 3, p 8, u read+write 48)", None),
         "divergence": (42.0 * unk, "42 B per unknown (u 24, mask 2, rhs 8, x 8)", None),

@@ -319,8 +319,9 @@ int mac_set_learned_smoothing(void* ctx, double omega);
  * reads the fine grid twice instead of four times; the CG iteration count may
  * rise. The preconditioner stays symmetric either way. prefetch = 1 runs the
  * V-cycle's first kernel as resident blocks that prefetch each next brick's CG
- * vectors with asynchronous bulk copies; 0 (default, measured faster on the
- * 256^3 pool and the 256x256x512 jet) runs one block per brick. */
+ * vectors with asynchronous bulk copies, and keeps the launch-by-launch solve for
+ * every size; 0 (default, measured faster on the 256^3 pool and the 256x256x512
+ * jet) gives each half brick a warp. */
 int mac_set_multigrid(void* ctx, int sweeps0, int prefetch);
 /* Launch of the pressure solve's CG-loop kernels (the V-cycle, SpMV, vector
  * updates and scalar finishers): on = 1 (default) launches each with
@@ -340,7 +341,9 @@ int mac_set_concurrent_binning(void* ctx, int on);
 /* The multigrid's dense levels (level 3, one cell per brick, and its
  * coarsenings): levels of more than max_cells cells (at least 64) run as
  * device-wide sweep kernels, the rest in one 1024-thread block that solves the
- * coarsest exactly. Default 1024. */
+ * coarsest exactly. A system whose level 3 is within max_cells is solved by one
+ * resident kernel (two sweeps, no prefetch; in the profile one region of
+ * MAC_PHASE_VCYCLE holds the whole solve). Default 1024. */
 int mac_set_coarse_block(void* ctx, int max_cells);
 /* The multigrid's smoother and coarse operators: weights w1, w2 of the two
  * Jacobi sweeps before and after each coarse correction (on every level), the
