@@ -396,6 +396,38 @@ __global__ void __launch_bounds__(128) k_conv_tile(ConvArgs a) {
   if (warp == 0) umma::tmem_dealloc(tmem, TCOLS);
 }
 
+// ------------------------------------------------ output layer, backward
+// The 1x1 layer has one real output channel, so the gradient of its input is one
+// product a channel (exact in FP32, hence the GEMM's value bit for bit), and as a
+// GEMM 15 of 16 K elements are zeros. A thread a voxel streams it, bound by
+// memory: 16 x 64^3 voxels 180 -> 51 us. (The forward pass stays with k_conv: a
+// sum in another order than tensor memory's moves the loss gradient's BF16
+// rounding.)
+__device__ __forceinline__ float2 bf2(uint32_t v) {
+  return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v));
+}
+
+// Zeroed where the input's activation (gate) is not positive.
+__global__ void __launch_bounds__(256) k_head_grad(const bf16* __restrict__ g, const bf16* __restrict__ wt,
+                                                   const bf16* __restrict__ gate, bf16* __restrict__ d, int V) {
+  const int v = blockIdx.x * 256 + threadIdx.x;
+  if (v >= V) return;
+  const float gv = __bfloat162float(g[(size_t)v * 16]);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint4 y = ldg16(gate + (size_t)v * 16 + 8 * h), w = ldg16(wt + 8 * h);
+    const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 b = bf2(ws[i]);
+      const __nv_bfloat162 r = __floats2bfloat162_rn(gv * b.x, gv * b.y);
+      o[i] = *reinterpret_cast<const uint32_t*>(&r);
+    }
+    *reinterpret_cast<uint4*>(d + (size_t)v * 16 + 8 * h) = gate8(make_uint4(o[0], o[1], o[2], o[3]), y);
+  }
+}
+
 // ------------------------------------------------ weight gradient (K = voxels)
 // dW[tap][co][ci] += sum_v in[v + off(tap)][ci] * g[v][co]; a CTA owns
 // 16 (tap, 8-channel group) row blocks = 128 GEMM rows and a range of voxels.
@@ -1781,7 +1813,9 @@ static int backward(Net& t, cudaStream_t st) {
   bf16** G = t.grad;
   int rc = cuda_ok(cudaMemsetAsync(t.g, 0, t.np * sizeof(float), st));
   rc |= bwd_w(t, 12, 0, src(A[D1], 16), none(), G[GOUT], st);
-  rc |= bwd_in(t, 12, 0, G[GOUT], G[D1], A[D1], 16, nullptr, st);
+  const int V = t.n * t.d * t.h * t.w;
+  k_head_grad<<<(V + 255) / 256, 256, 0, st>>>(G[GOUT], t.wb + t.woff[12], A[D1], G[D1], V);
+  ++t.launches;
   rc |= bwd_w(t, 11, 0, src(A[C1], 16), none(), G[D1], st);
   rc |= bwd_in(t, 11, 0, G[D1], G[C1], A[C1], 16, nullptr, st);
   rc |= bwd_w(t, 10, 0, src(A[S1], 16), src(A[U1], 16, 1), G[C1], st);
