@@ -20,7 +20,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -1633,7 +1632,7 @@ static int copy_host(Net& t, const HostCopy* list, int n, bool up) {
   try {
     for (; made < kCopyLanes - 1; ++made)
       lanes[made] = std::thread([&, l = made + 1] { rcs[l] = copy_lane(t, list, n, up, l); });
-  } catch (const std::system_error&) {  // no thread to be had: this one does the rest
+  } catch (...) {  // no thread to be had (or no memory for one): this one does the rest
   }
   rcs[0] = copy_lane(t, list, n, up, 0);
   for (int l = made + 1; l < kCopyLanes; ++l) rcs[l] = copy_lane(t, list, n, up, l);
