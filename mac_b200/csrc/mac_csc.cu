@@ -238,9 +238,12 @@ int csc_cg_resident(cudaStream_t st, int n, const int* off, const int* ind, cons
 
 // flags (zeroed before): [0] the matrix is not symmetric with exactly one
 // negative diagonal entry a column (or its arrays are not valid), [1] a column
-// of more than kCgRow entries, [2] a column repeats a row, so that the entry by
-// entry comparison decides nothing. Column i is scanned linearly for the
-// mirror entry (the reference's columns hold at most 7).
+// of more than kCgRow entries, [2] (REPEATS only) a column repeats a row, so that
+// the entry by entry comparison decides nothing. Column i is scanned linearly for the
+// mirror entry (the reference's columns hold at most 7). The search for repeats
+// takes the square of a column's length, so only the caller that acts on it
+// asks for it, for columns whose length it has bounded.
+template <bool REPEATS>
 __global__ void k_csc_check(int n, const int* __restrict__ off, const int* __restrict__ ind,
                             const double* __restrict__ val, double* flags) {
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
@@ -264,12 +267,15 @@ __global__ void k_csc_check(int n, const int* __restrict__ off, const int* __res
             break;
           }
         if (!found) bad = true;
-        for (int m = k0; m < k; ++m)
-          if (ind[m] == i) flags[2] = 1.0;
+        if (REPEATS)
+          for (int m = k0; m < k; ++m)
+            if (ind[m] == i) flags[2] = 1.0;
       }
     }
     if (bad || ndiag != 1) flags[0] = 1.0;
   }
 }
+template __global__ void k_csc_check<false>(int, const int*, const int*, const double*, double*);
+template __global__ void k_csc_check<true>(int, const int*, const int*, const double*, double*);
 
 }  // namespace mac

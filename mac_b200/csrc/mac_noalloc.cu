@@ -28,6 +28,7 @@ __global__ void k_csc_diag(int n, const int* __restrict__ off, const int* __rest
 __global__ void k_csc_vec(int n, int mode, const double* b, double* x, double* r, double* z, double* p,
                           const double* q, const double* dinv, double* scal, double a);
 // Defined with the resident solve (mac_csc.cu).
+template <bool REPEATS>
 __global__ void k_csc_check(int n, const int* __restrict__ off, const int* __restrict__ ind,
                             const double* __restrict__ val, double* flags);
 
@@ -78,7 +79,7 @@ static int csc_solve_noalloc(cudaStream_t st, int n, const int* off, const int* 
   if (g > 1184) g = 1184;
   double hs[8];
   if ((rc = check(cudaMemsetAsync(scal, 0, 64, st)))) return rc;
-  k_csc_check<<<g, 256, 0, st>>>(n, off, ind, val, scal);
+  k_csc_check<false><<<g, 256, 0, st>>>(n, off, ind, val, scal);
   // the resident solve runs right behind the check and returns at once when
   // the check refused the matrix or found a longer row: one host read in all
   int enqueued = 0;

@@ -521,6 +521,7 @@ static int csc_reserve(Ctx* c, int n, int nnz, size_t nvec, int** off, int** ind
   return MAC_OK;
 }
 
+template <bool REPEATS>
 __global__ void k_csc_check(int n, const int* __restrict__ off, const int* __restrict__ ind,
                             const double* __restrict__ val, double* flags);
 
@@ -548,7 +549,7 @@ static int csc_factorize(Ctx* c, int n, const int* offset, const int* indice, co
     double f[4];
     rc = check(cudaMemsetAsync(c->csc_vec, 0, 32, st));
     if (rc) return rc;
-    k_csc_check<<<std::min(grid_for(n, 256), 1184), 256, 0, st>>>(n, c->csc_off, c->csc_ind, c->csc_val,
+    k_csc_check<true><<<std::min(grid_for(n, 256), 1184), 256, 0, st>>>(n, c->csc_off, c->csc_ind, c->csc_val,
                                                                   c->csc_vec); MAC_COUNT(c);
     rc = check(cudaGetLastError());
     if (!rc) rc = check(cudaMemcpyAsync(f, c->csc_vec, 32, cudaMemcpyDeviceToHost, st));
