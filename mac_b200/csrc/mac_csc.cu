@@ -242,7 +242,7 @@ int csc_cg_resident(cudaStream_t st, int n, const int* off, const int* ind, cons
 // the entry by entry comparison decides nothing. Column i is scanned linearly for the
 // mirror entry (the reference's columns hold at most 7). The search for repeats
 // takes the square of a column's length, so only the caller that acts on it
-// asks for it, for columns whose length it has bounded.
+// asks for it, for valid arrays and columns whose length it has bounded.
 template <bool REPEATS>
 __global__ void k_csc_check(int n, const int* __restrict__ off, const int* __restrict__ ind,
                             const double* __restrict__ val, double* flags) {
@@ -267,11 +267,14 @@ __global__ void k_csc_check(int n, const int* __restrict__ off, const int* __res
             break;
           }
         if (!found) bad = true;
-        if (REPEATS)
-          for (int m = k0; m < k; ++m)
-            if (ind[m] == i) flags[2] = 1.0;
       }
     }
+    // all pairs of the column, whatever the comparison met: a coupling in unequal
+    // parts differs from its mirror's first part and is equal all the same
+    if (REPEATS)
+      for (int k = k0 + 1; k < k1; ++k)
+        for (int m = k0; m < k; ++m)
+          if (ind[m] == ind[k]) flags[2] = 1.0;
     if (bad || ndiag != 1) flags[0] = 1.0;
   }
 }

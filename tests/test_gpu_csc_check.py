@@ -44,3 +44,33 @@ def test_long_column_costs_its_length():
     res[1:] += 1e-3 * got[0]
     assert np.linalg.norm(res - b) <= 1e-11 * np.linalg.norm(b)
     assert t[0].elapsed_time(t[1]) < 500.0
+
+
+@pytest.mark.parametrize("split", ["one coupling", "all couplings"])
+def test_unequal_parts_of_a_coupling_stay_with_cg(split):
+    """Couplings stored as v / 4 and 3 v / 4 in one column and the other way round
+    in its mirror: the same entries, so the matrix is symmetric and CG solves it,
+    in the iterations of the matrix with whole entries (the parts add up exactly,
+    up to the order of a row's sum)."""
+    from test_gpu_csc_resident import _ctx, _laplacian
+    A = _laplacian((9, 10, 11), 0.05)
+    n = A.shape[0]
+    off, ind, val = [0], [], []
+    for j in range(n):
+        for k in range(A.indptr[j], A.indptr[j + 1]):
+            i, v = int(A.indices[k]), A.data[k]
+            if i != j and (split == "all couplings" or {i, j} == {0, 1}):
+                parts = [0.25 * v, 0.75 * v]
+                ind += [i, i]
+                val += parts if i < j else parts[::-1]
+            else:
+                ind.append(i)
+                val.append(v)
+        off.append(len(ind))
+    b = np.random.default_rng(2).uniform(-1, 1, n)
+    with _ctx() as ctx:
+        want = ctx.csc_solve(A.indptr, A.indices, A.data, b)
+        its = ctx.stats()["iterations"]
+        got = ctx.csc_solve(np.array(off), np.array(ind), np.array(val), b)
+        assert abs(ctx.stats()["iterations"] - its) <= 1
+    assert np.linalg.norm(got - want) <= 1e-8 * np.linalg.norm(want)
