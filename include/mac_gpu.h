@@ -345,6 +345,10 @@ int mac_set_concurrent_binning(void* ctx, int on);
  * resident kernel (two sweeps, no prefetch; in the profile one region of
  * MAC_PHASE_VCYCLE holds the whole solve). Default 1024. */
 int mac_set_coarse_block(void* ctx, int max_cells);
+/* Polls after which a wait inside the drop-in CSC solve, for a value that another
+ * thread block publishes, gives up and the call returns MAC_ERR_TIMEOUT. Default
+ * 2^22 (seconds). */
+int mac_set_wait_limit(void* ctx, int polls);
 /* The multigrid's smoother and coarse operators: weights w1, w2 of the two
  * Jacobi sweeps before and after each coarse correction (on every level), the
  * weight of the single finest-level sweep (mac_set_multigrid(ctx, 1, .)), and

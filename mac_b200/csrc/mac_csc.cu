@@ -19,7 +19,7 @@ namespace mac {
 constexpr int kCgThreads = 512;
 constexpr int kCgRow = kCscRow;      // entries of a row held in registers (the 7-point stencil)
 constexpr int kCgMaxBlocks = 512;    // blocks whose slots one block's threads can poll
-constexpr int kCgSpin = 1 << 22;     // polls before a wait gives up (seconds)
+constexpr int kCgSpin = kWaitPolls;  // polls before a wait for the other blocks gives up
 // Each block's slot has a 128-byte line to itself: with 32-byte slots the
 // polls of one line by all blocks queued behind each other (an exchange among
 // 148 blocks took 2.4 us, against 1.0 us with a line each).
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(kCgThreads, MINB) k_csc_cg(int n, const int* _
                                                              const double* __restrict__ bv, double* x,
                                                              unsigned long long* z, unsigned long long* slots,
                                                              const double* flags, double rtol2, int max_iters,
-                                                             double* out) {
+                                                             int polls, double* out) {
   if (flags && (flags[0] != 0.0 || flags[1] != 0.0)) return;
   const int j = blockIdx.x * kCgThreads + threadIdx.x;
   const bool live = j < n;
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(kCgThreads, MINB) k_csc_cg(int n, const int* _
     // the neighbours' p = z + beta p, formed here as their own row forms it
     double q = 0;
     bool got = false;
-    for (int i = 0; i < kCgSpin && !got; ++i) {
+    for (int i = 0; i < polls && !got; ++i) {
       double zn[kCgRow];
       got = true;
 #pragma unroll
@@ -177,9 +177,10 @@ __global__ void __launch_bounds__(kCgThreads, MINB) k_csc_cg(int n, const int* _
           q += av[m] * pn[m];
         }
     }
-    q = got ? -q : __longlong_as_double(0x7ff8000000000000ll);  // M = -A; a wait that ran out ends the solve
+    // M = -A; the NaN of a wait that ran out ends every block's solve
+    q = got ? -q : __longlong_as_double(0x7ff8000000000000ll);
     s0 = p * q;
-    ok = grid_sum<false>(s0, s1, slots, ++tag);
+    ok = grid_sum<false>(s0, s1, slots, ++tag) && got;
     // breakdown: x keeps the last finite iterate
     if (!ok || !(s0 != 0.0 && isfinite(s0))) break;
     const double alpha = rz / s0;
@@ -205,18 +206,19 @@ __global__ void __launch_bounds__(kCgThreads, MINB) k_csc_cg(int n, const int* _
     out[1] = rr;
     out[2] = bb;
   }
-  if (threadIdx.x == 0 && !ok) out[3] = 1.0;
+  if (!ok) out[3] = 1.0;
 }
 
 // Enqueues the whole solve of A x = b (A symmetric with a negative diagonal,
 // rows of at most kCgRow entries) on st: `work` (16-byte aligned) holds 2 n
 // doubles of tagged z and kCscWork more, res (4 doubles) receives iterations,
-// r.r, b.b and a timeout mark. *enqueued = 0 when the system does not fit the
-// resident form: a row a thread and two blocks an SM hold 151,552 rows on 148
-// SMs, and a block polls at most kCgMaxBlocks slots.
+// r.r, b.b and a timeout mark; polls bounds the wait for a neighbour's z.
+// *enqueued = 0 when the system does not fit the resident form: a row a thread
+// and two blocks an SM hold 151,552 rows on 148 SMs, and a block polls at most
+// kCgMaxBlocks slots.
 int csc_cg_resident(cudaStream_t st, int n, const int* off, const int* ind, const double* val, const double* b,
-                    double* x, double* work, const double* flags, double rtol, int max_iters, double* res,
-                    int* enqueued) {
+                    double* x, double* work, const double* flags, double rtol, int max_iters, int polls,
+                    double* res, int* enqueued) {
   *enqueued = 0;
   int dev = 0, nsm = 0, occ = 0, coop = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) ||
@@ -230,7 +232,7 @@ int csc_cg_resident(cudaStream_t st, int n, const int* off, const int* ind, cons
   if (!rc) rc = check(cudaMemsetAsync(res, 0, 32, st));
   if (rc) return rc;
   double rtol2 = rtol * rtol;
-  void* args[] = {&n, &off, &ind, &val, &b, &x, &z, &slots, &flags, &rtol2, &max_iters, &res};
+  void* args[] = {&n, &off, &ind, &val, &b, &x, &z, &slots, &flags, &rtol2, &max_iters, &polls, &res};
   rc = check(cudaLaunchCooperativeKernel(g <= nsm ? (const void*)k_csc_cg<1> : (const void*)k_csc_cg<2>, dim3(g), dim3(kCgThreads), args, 0, st));
   if (!rc) *enqueued = 1;
   return rc;

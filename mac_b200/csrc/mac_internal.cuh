@@ -42,6 +42,8 @@ enum ErrBits : int {
   kErrTimeout = 16,  // a bounded wait on an asynchronous copy ran out
 };
 
+constexpr int kWaitPolls = 1 << 22;  // polls after which a resident solve's wait gives up (seconds)
+
 // Field indices of the FP64 per-cell block.
 enum F64 : int { U0X = 0, U0Y, U0Z, U1X, U1Y, U1Z, AX, AY, AZ, PRES, NF64 };
 
@@ -208,6 +210,7 @@ struct Ctx {
   int res_grid = 0;           // blocks of the resident solve (0: not available)
   int res_smem = 0;           // its largest dynamic shared memory
   int res_cluster = 0;        // one cluster of 16 of its blocks fits
+  int wait_polls = kWaitPolls;  // of the CSC solve's wait for a neighbour's value
   int bulk_grid = 0;          // its grid (blocks resident on all SMs at once)
   int npart_head = 0;         // partial sums the V-cycle's first kernel left (its grid)
   int npart_tail = 0;         // and its last
@@ -605,7 +608,7 @@ void csc_release(Ctx* c, size_t keep);
 constexpr int kCscRow = 7;
 constexpr size_t kCscWork = 2 * 16 * 512;
 int csc_cg_resident(cudaStream_t st, int n, const int* off, const int* ind, const double* val, const double* b,
-                    double* x, double* work, const double* flags, double rtol, int max_iters, double* res,
-                    int* enqueued);
+                    double* x, double* work, const double* flags, double rtol, int max_iters, int polls,
+                    double* res, int* enqueued);
 
 }  // namespace mac

@@ -84,7 +84,8 @@ static int csc_solve_noalloc(cudaStream_t st, int n, const int* off, const int* 
   // the check refused the matrix or found a longer row: one host read in all
   int enqueued = 0;
   static_assert(kNoAllocSlots >= 2 * (size_t)MAC_NOALLOC_MAX_N + kCscWork, "z and the exchange slots fit the scratch");
-  if ((rc = csc_cg_resident(st, n, off, ind, val, b, x, v, scal, rtol, max_iters, scal + 4, &enqueued))) return rc;
+  if ((rc = csc_cg_resident(st, n, off, ind, val, b, x, v, scal, rtol, max_iters, kWaitPolls, scal + 4, &enqueued)))
+    return rc;
   if ((rc = check(cudaGetLastError())) || (rc = read_slots(hs, scal, st))) return rc;
   if (hs[0] != 0.0) return MAC_ERR_MATRIX;
   if (enqueued && hs[1] == 0.0) {

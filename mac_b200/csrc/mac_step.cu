@@ -209,7 +209,7 @@ static int csc_solve_cg(Ctx* c, const double* hb, double* hx) {
     int rc = check(cudaMemcpyAsync(b, hb, 8 * (size_t)n, cudaMemcpyHostToDevice, st)), enqueued = 0;
     if (!rc)
       rc = csc_cg_resident(st, n, c->csc_off, c->csc_ind, c->csc_val, b, x, v, nullptr, c->prm.rtol, c->prm.max_iters,
-                           res, &enqueued);
+                           c->wait_polls, res, &enqueued);
     if (rc) return rc;
     if (enqueued) {
       MAC_COUNT(c);
@@ -707,6 +707,13 @@ int mac_set_coarse_block(void* ctx, int max_cells) {
   if (max_cells < 64) return MAC_ERR_INVALID;
   c->blk_max_cells = max_cells;
   c->system_ready = false;  // the level split is made with the system
+  return MAC_OK;
+}
+
+int mac_set_wait_limit(void* ctx, int polls) {
+  CTX_OR_FAIL();
+  if (polls < 0) return MAC_ERR_INVALID;
+  c->wait_polls = polls;
   return MAC_OK;
 }
 
