@@ -345,9 +345,11 @@ int mac_set_concurrent_binning(void* ctx, int on);
  * resident kernel (two sweeps, no prefetch; in the profile one region of
  * MAC_PHASE_VCYCLE holds the whole solve). Default 1024. */
 int mac_set_coarse_block(void* ctx, int max_cells);
-/* Polls after which a wait inside the drop-in CSC solve, for a value that another
- * thread block publishes, gives up and the call returns MAC_ERR_TIMEOUT. Default
- * 2^22 (seconds). */
+/* Polls after which a wait inside a one-launch solve gives up and the call returns
+ * MAC_ERR_TIMEOUT: in the pressure solve for the other thread blocks, in the
+ * drop-in CSC solve for a value that another block publishes. Default 2^22
+ * (seconds). After a timeout of the pressure solve the context returns the same
+ * status until the next mac_upload_state. */
 int mac_set_wait_limit(void* ctx, int polls);
 /* The multigrid's smoother and coarse operators: weights w1, w2 of the two
  * Jacobi sweeps before and after each coarse correction (on every level), the

@@ -395,6 +395,8 @@ static int upload(Ctx* c, const mac_host_state* s) {
   h.dt = s->dt;
   h.t = s->t;
   std::memcpy(c->hs, &h, sizeof(h));
+  // the error bits go, and with them what a timed-out solve left of its barrier
+  MAC_CUDA(cudaMemsetAsync(c->res_slots, 0, 8 * kResSlots, st));
   MAC_CUDA(cudaMemcpyAsync(c->ds, c->hs, sizeof(Scalars), cudaMemcpyHostToDevice, st));
   c->seed = s->step;
   c->nlive_host = nb;

@@ -39,7 +39,7 @@ enum ErrBits : int {
   kErrParticles = 2,
   kErrHash = 4,
   kErrPending = 8,
-  kErrTimeout = 16,  // a bounded wait on an asynchronous copy ran out
+  kErrTimeout = 16,  // a bounded wait ran out: on an asynchronous copy, or of a resident solve's blocks for each other
 };
 
 constexpr int kWaitPolls = 1 << 22;  // polls after which a resident solve's wait gives up (seconds)
@@ -210,7 +210,7 @@ struct Ctx {
   int res_grid = 0;           // blocks of the resident solve (0: not available)
   int res_smem = 0;           // its largest dynamic shared memory
   int res_cluster = 0;        // one cluster of 16 of its blocks fits
-  int wait_polls = kWaitPolls;  // of the CSC solve's wait for a neighbour's value
+  int wait_polls = kWaitPolls;  // of the resident solve's wait for its blocks, and of the CSC solve's for a neighbour's value
   int bulk_grid = 0;          // its grid (blocks resident on all SMs at once)
   int npart_head = 0;         // partial sums the V-cycle's first kernel left (its grid)
   int npart_tail = 0;         // and its last

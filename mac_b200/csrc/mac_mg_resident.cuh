@@ -22,7 +22,6 @@ constexpr int kResThreads = 512;                 // 128 registers a thread (spil
 constexpr int kResGroups = kResThreads / 128;    // bricks a block works on at once
 constexpr int kResWarps = kResThreads / 32;
 constexpr int kResCluster = 16;                  // blocks of the one-cluster form
-constexpr int kResSpin = 1 << 22;
 
 template <class T>
 struct ResArgs {
@@ -42,6 +41,7 @@ struct ResArgs {
   Params P;
   double rtol2;
   int max_iters;
+  int polls;         // after which a wait for the other blocks gives up
   size_t blk_bytes;  // shared memory of block 0's levels
   int cluster;       // 1: launched as one cluster
 };
@@ -59,6 +59,7 @@ struct ResSync {
   unsigned target;
   unsigned parity;
   int cluster;
+  int polls;
   double* red;         // [kResWarps] warp sums, then [2][kResCluster] the cluster's slots (grid: the total)
   int* ok;
 };
@@ -116,7 +117,7 @@ __device__ __forceinline__ bool res_wait(ResSync& y, double* sum) {
   if (w == 0) {
     if (lane == 0) {
       bool ok = false;
-      for (int i = 0; i < kResSpin && !ok; ++i) {
+      for (int i = 0; i < y.polls && !ok; ++i) {
         unsigned v;
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(y.counter) : "memory");
         ok = (int)(v - y.target) >= 0;
@@ -747,7 +748,12 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const __grid_con
   double* st64 = reinterpret_cast<double*>(res_smem) + (threadIdx.x >> 7) * kS1;
   T* st = reinterpret_cast<T*>(st64);
   Scalars* ds = A.ds;
-  if (ds->done) return;
+  // After a wait that ran out the count of arrivals is off until the next upload
+  // clears it together with the mark. One thread asks: a block of this launch may
+  // set the mark meanwhile.
+  if (threadIdx.x == 0) sok = ds->done || (ds->err & kErrTimeout);
+  __syncthreads();
+  if (sok) return;
   const int nd = A.nd, G = gridDim.x;
   const T w1 = (T)A.P.mgw1, w2 = (T)A.P.mgw2;
   double* sinv = reinterpret_cast<double*>(res_smem + kResStage);
@@ -759,11 +765,12 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const __grid_con
     if (exact) blk_copy(sinv, A.inv, (int64_t)SL[nl - 1].n * 64);
   }
   // the count goes on from the last solve's, so nothing is cleared: what it was
-  // then is kept beside it (block 0 writes it once every block has read it)
+  // then is kept beside it (block 0 writes it once every block has read it). Blocks
+  // that give up leave at different counts: no solve starts from there (above).
   unsigned* counter = reinterpret_cast<unsigned*>(A.slots);
   unsigned* last = counter + 32;
   __syncthreads();
-  ResSync y{counter, reinterpret_cast<double*>(A.slots + 32), *last, 0u, A.cluster, red, &sok};
+  ResSync y{counter, reinterpret_cast<double*>(A.slots + 32), *last, 0u, A.cluster, A.polls, red, &sok};
   // bricks by group and cells by warp, dealt to the blocks in turn, so that a
   // system smaller than the grid still spreads over every SM
   const int j0 = (threadIdx.x >> 7) * G + blockIdx.x, dj = G * kResGroups;
@@ -989,6 +996,7 @@ static int cg_resident_t(Ctx* c, int* enqueued) {
   A.P = c->dp;
   A.rtol2 = c->prm.rtol * c->prm.rtol;
   A.max_iters = c->prm.max_iters;
+  A.polls = c->wait_polls;
   A.cluster = nd <= kResClusterBricks && c->res_cluster ? 1 : 0;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];

@@ -469,7 +469,7 @@ class Context:
         self._check(self.lib.mac_set_coarse_block(self.h, int(max_cells)), "mac_set_coarse_block")
 
     def set_wait_limit(self, polls=1 << 22):
-        """Polls after which a wait inside the CSC solve gives up (MacError -7)."""
+        """Polls after which a wait inside a one-launch solve gives up (MacError -7)."""
         self._check(self.lib.mac_set_wait_limit(self.h, int(polls)), "mac_set_wait_limit")
 
     def set_concurrent_binning(self, on=True):
