@@ -213,9 +213,9 @@ __global__ void __launch_bounds__(kCgThreads, MINB) k_csc_cg(int n, const int* _
 // rows of at most kCgRow entries) on st: `work` (16-byte aligned) holds 2 n
 // doubles of tagged z and kCscWork more, res (4 doubles) receives iterations,
 // r.r, b.b and a timeout mark; polls bounds the wait for a neighbour's z.
-// *enqueued = 0 when the system does not fit the resident form: a row a thread
-// and two blocks an SM hold 151,552 rows on 148 SMs, and a block polls at most
-// kCgMaxBlocks slots.
+// *enqueued = 0 when the driver refuses the launch or the system does not fit the
+// resident form: a row a thread and two blocks an SM hold 151,552 rows on 148
+// SMs, and a block polls at most kCgMaxBlocks slots.
 int csc_cg_resident(cudaStream_t st, int n, const int* off, const int* ind, const double* val, const double* b,
                     double* x, double* work, const double* flags, double rtol, int max_iters, int polls,
                     double* res, int* enqueued) {
@@ -233,9 +233,17 @@ int csc_cg_resident(cudaStream_t st, int n, const int* off, const int* ind, cons
   if (rc) return rc;
   double rtol2 = rtol * rtol;
   void* args[] = {&n, &off, &ind, &val, &b, &x, &z, &slots, &flags, &rtol2, &max_iters, &polls, &res};
-  rc = check(cudaLaunchCooperativeKernel(g <= nsm ? (const void*)k_csc_cg<1> : (const void*)k_csc_cg<2>, dim3(g), dim3(kCgThreads), args, 0, st));
-  if (!rc) *enqueued = 1;
-  return rc;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  cfg.gridDim = g;
+  cfg.blockDim = kCgThreads;
+  cfg.stream = st;
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  launch_resident(cfg, g <= nsm ? (const void*)k_csc_cg<1> : (const void*)k_csc_cg<2>, args, enqueued);
+  return MAC_OK;
 }
 
 // flags (zeroed before): [0] the matrix is not symmetric with exactly one

@@ -327,6 +327,16 @@ inline void launch_k(const Ctx* c, void (*k)(P...), dim3 grid, dim3 block, size_
   launch_on(c, c->stream, k, grid, block, smem, static_cast<A&&>(args)...);
 }
 
+// Launches a kernel whose blocks must all be resident at once. *enqueued = 0 when
+// the driver does not take it (an SM share smaller than the device's attributes
+// say, a cluster that does not fit beside other work): the caller's form of
+// separate launches does the work then. An error of earlier work is not lost, the
+// next check meets it again.
+inline void launch_resident(const cudaLaunchConfig_t& cfg, const void* k, void** args, int* enqueued) {
+  *enqueued = cudaLaunchKernelExC(&cfg, k, args) == cudaSuccess;
+  if (!*enqueued) cudaGetLastError();
+}
+
 // ---------------------------------------------------------------- helpers
 __host__ __device__ inline unsigned long long pack_key(int x, int y, int z) {
   return ((unsigned long long)((uint32_t)(x + (1 << 20)) & 0x1FFFFFu)) |

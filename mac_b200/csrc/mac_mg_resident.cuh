@@ -1017,10 +1017,9 @@ static int cg_resident_t(Ctx* c, int* enqueued) {
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;
   }
-  int rc = check(cudaLaunchKernelEx(&cfg, k_cg_resident<T>, A));
-  if (rc) return rc;
-  MAC_COUNT(c);
-  *enqueued = 1;
+  void* args[] = {&A};
+  launch_resident(cfg, (const void*)k_cg_resident<T>, args, enqueued);
+  if (*enqueued) MAC_COUNT(c);
   return MAC_OK;
 }
 
