@@ -1040,10 +1040,17 @@ int cg_resident(Ctx* c, int* enqueued) {
 // What a device offers the resident form: its blocks (one an SM), dynamic
 // shared memory, and whether a cluster of kResCluster blocks fits. Asked once a
 // device (the questions take half a millisecond, and a context is made for each
-// world).
+// world). The kernel's attributes are set for each context: a reset of the device
+// by the host program takes them back.
 struct ResDevice {
   int asked = 0, grid = 0, smem = 0, cluster = 0;
 };
+
+template <class T>
+static int res_allow(int smem) {
+  int rc = check(cudaFuncSetAttribute(k_cg_resident<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  return rc ? rc : check(cudaFuncSetAttribute(k_cg_resident<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+}
 
 template <class T>
 static int res_ask(ResDevice& d, int dev, int nsm, int optin) {
@@ -1051,8 +1058,7 @@ static int res_ask(ResDevice& d, int dev, int nsm, int optin) {
   int rc = check(cudaFuncGetAttributes(&fa, k_cg_resident<T>));
   if (rc) return rc;
   d.smem = optin - (int)fa.sharedSizeBytes;
-  rc = check(cudaFuncSetAttribute(k_cg_resident<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, d.smem));
-  if (!rc) rc = check(cudaFuncSetAttribute(k_cg_resident<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  rc = res_allow<T>(d.smem);
   int occ = 0, coop = 0, ncl = 0;
   if (!rc) rc = check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_cg_resident<T>, kResThreads, d.smem));
   if (!rc) rc = check(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
@@ -1082,10 +1088,8 @@ static int res_configure_t(Ctx* c, int nsm, int optin) {
   ResDevice own, *d = &own;
   std::lock_guard<std::mutex> lock(mu);
   if (c->prm.device < kDevices) d = &known[c->prm.device];
-  if (!d->asked) {
-    int rc = res_ask<T>(*d, c->prm.device, nsm, optin);
-    if (rc) return rc;
-  }
+  int rc = d->asked ? res_allow<T>(d->smem) : res_ask<T>(*d, c->prm.device, nsm, optin);
+  if (rc) return rc;
   c->res_grid = d->grid;
   c->res_smem = d->smem;
   c->res_cluster = d->cluster;

@@ -1,4 +1,6 @@
-"""A device that refuses the launch of a one-launch solve (blocks that do not fit
+"""What a one-launch solve needs from the runtime, and what is done without it.
+
+A device that refuses the launch of a one-launch solve (blocks that do not fit
 together: a share of the SMs, other work in the way): the call goes on with its
 separate launches. The refusal comes from a stand-in for the runtime's launch
 calls, preloaded into a child process, that returns
@@ -84,3 +86,26 @@ def test_refused_launches_take_the_separate_ones(tmp_path):
         assert np.linalg.norm(plain[k] - refused[k]) <= 1e-8 * np.linalg.norm(plain[k]), k
     for n in (17, 63):
         assert refused["launches%d" % n] > plain["launches%d" % n]
+
+
+RESET = r"""
+import ctypes, sys
+import numpy as np
+sys.path.insert(0, sys.argv[1] + "/tests")
+sys.path.insert(0, sys.argv[1])
+from test_gpu_resident_solve import _solve, _world
+s = _world(63, 0.5)
+a, sa, la = _solve(s, "mgpcg64", False)
+cudart = next(l.split()[-1] for l in open("/proc/self/maps") if "libcudart.so" in l)
+assert ctypes.CDLL(cudart).cudaDeviceReset() == 0
+b, sb, lb = _solve(s, "mgpcg64", False)
+assert (la, sa["iterations"]) == (lb, sb["iterations"]), (la, lb)
+assert np.array_equal(a.f64["p"], b.f64["p"])
+"""
+
+
+def test_device_reset_by_the_host_program():
+    """The kernel's shared memory and cluster size are allowed again for a context
+    made after the reset: the solve is one launch as before."""
+    r = subprocess.run([sys.executable, "-c", RESET, ROOT], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
