@@ -267,8 +267,6 @@ __global__ void k_compact_particles_done(Scalars* ds) {
 // ------------------------------------------------ Create_Fluid_Particle
 // Same jitter as the oracle's restatement: splitmix64 over (seed, key, slot, axis).
 __device__ inline unsigned long long mix64(unsigned long long z) {
-  pdl_entry();
-  pdl_entry();
   z += 0x9E3779B97F4A7C15ull;
   z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
   z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
@@ -547,7 +545,6 @@ __global__ void __launch_bounds__(512) k_depth_relax(const int* __restrict__ bli
 // (SetInterior: always) otherwise; the seeds keep their material.
 __global__ void k_depth_types(const int* __restrict__ blist, const int8_t* __restrict__ lay,
                               const int16_t* __restrict__ depth, uint8_t* type, Params P, Scalars* ds) {
-  pdl_entry();
   pdl_entry();
   int n = ds->nlive;
   for (int bi = blockIdx.x; bi < n; bi += gridDim.x) {
