@@ -203,6 +203,7 @@ class HostState:
             f64 = lambda n: np.empty(n, np.float64)
             u8 = lambda n: np.empty(n, np.uint8)
             i32 = lambda n: np.empty(n, np.int32)
+        self.pinned, self.stage_buffers = pinned, stage_buffers
         self.nbricks, self.nparticles = nbricks, nparticles
         self.cap_bricks, self.cap_particles = nbricks, nparticles
         self.keys = i32(3 * max(nbricks, 1))
@@ -216,6 +217,12 @@ class HostState:
         self.pos = f64(3 * max(nparticles, 1))
         self.t = self.dt = 0.0
         self.step = 0
+
+    def grown(self, nbricks: int, nparticles: int) -> "HostState":
+        """A HostState of the same layout (pinned, depth, stage buffers) with room
+        for at least this many bricks and particles; the content is not copied."""
+        return HostState(max(nbricks, self.cap_bricks), max(nparticles, self.cap_particles), pinned=self.pinned,
+                         depth=self.depth is not None, stage_buffers=self.stage_buffers)
 
     def fill(self, s: State) -> "HostState":
         nb, nc = s.nbricks, s.nbricks * BRICK_CELLS
@@ -321,12 +328,15 @@ class Context:
 
     def download(self, host: HostState | None = None, to_state: bool = True):
         """Reads the device state through mac_download_state into ``host`` (a
-        new HostState if it is missing or too small). Returns it as a State
+        new HostState if it is missing, one of the same layout with more room if
+        it is too small). Returns it as a State
         (key-sorted copies of the arrays), or, with ``to_state=False``, the
         HostState itself with the arrays as the C-ABI wrote them."""
         nb, npart = self.sizes()
-        if host is None or host.cap_bricks < nb or host.cap_particles < npart:
+        if host is None:
             host = HostState(nb, npart, depth=bool(self.params.depth_mode))
+        elif host.cap_bricks < nb or host.cap_particles < npart:
+            host = host.grown(nb, npart)
         host.nbricks, host.nparticles = nb, npart
         st = host.c_struct()
         self._check(self.lib.mac_download_state(self.h, ctypes.byref(st)), "mac_download_state")
