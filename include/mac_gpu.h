@@ -302,7 +302,7 @@ int mac_unet_time_forward(void* net, int n, int d, int h, int w, int reps, doubl
  * tile's input planes (weight gradient: lines) with their halo in shared memory
  * once and run the 27 taps from them; 0 gather every tap's operand separately.
  * Both accumulate in the same order (the weight gradient on grids whose width is
- * a multiple of 16). */
+ * a multiple of 16, elsewhere 1 adds up shorter sums). */
 int mac_unet_set_conv(void* net, int staged);
 
 /* Attaches a network (mac_unet_create) as the preconditioner of the

@@ -769,7 +769,7 @@ __global__ void __launch_bounds__(128, March<KC, NC>::occ) k_conv_march(ConvArgs
 // --------------------------------------- 3x3x3 weight gradient from staged lines
 // dW[tap][co][ci] += sum_v in[v + off(tap)][ci] * g[v][co]. A CTA takes
 // one group of eight input channels and a range of voxels v in linear order (the
-// ranges k_wgrad takes) and walks the input lines they touch, L whole x-lines of
+// ranges k_wgrad takes, or shorter: wgrad_lines_t) and walks the input lines they touch, L whole x-lines of
 // one plane a step, keeping its products in one tensor-memory accumulator of 128
 // rows x 3 COUT columns until the end. Row blocks j = 3 (dy + 1) + dx + 1 = 0..8
 // are the nine in-plane taps (rows 72.. are not used): a line is staged in three
@@ -791,6 +791,7 @@ constexpr int kWlLoad = 512;  // loading threads; a further warp issues the MMAs
 constexpr int kWlIn = 2;      // chunks of input lines a thread carries
 constexpr int kWlVox = 256;   // voxels of a step, padding included
 constexpr int kWlPad = 16;    // bytes between copies: row blocks start in different banks
+constexpr int kWlMinW = 9;    // narrowest line
 constexpr int kWlMaxW = kWlVox / 2;  // widest line: one of COUT = 64 is a whole step
 static_assert(4 * (kWlMaxW + 2) <= kWlLoad * kWlIn, "the lines of the widest step fit the threads' chunks");
 
@@ -1453,8 +1454,15 @@ static int wgrad_range(int cin, int taps, long V) {
 template <int COUT>
 static void wgrad_lines_t(int cin, WgradArgs a, cudaStream_t st) {
   const long V = (long)a.n * a.d * a.h * a.w;
+  const int w16 = (a.w + 15) / 16 * 16;
   a.vox_per_cta = wgrad_range(cin, 27, V);
-  const int L = wl_vox<COUT>() / ((a.w + 15) / 16 * 16), smem = 2 * wl_stage<COUT>(a.w, L);
+  // Padded lines take w16 / w times the MMAs for the same voxels, each of which
+  // truncates the sum it adds to: whole lines, at most half as many MMAs a sum as
+  // k_wgrad's range has. Error against 64 bits in multiples of k_wgrad's, with its
+  // ranges and with these: lines of 40 (16 columns) 1.0 and 0.35, of 20 (32 columns)
+  // 1.1 and 0.24, of 10 (64 columns) 1.4 and 0.4. The times are the same.
+  if (a.w % 16) a.vox_per_cta = std::max(1, a.vox_per_cta / (2 * w16)) * a.w;
+  const int L = wl_vox<COUT>() / w16, smem = 2 * wl_stage<COUT>(a.w, L);
   cudaFuncSetAttribute(k_wgrad_lines<COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   k_wgrad_lines<COUT><<<dim3((unsigned)((V + a.vox_per_cta - 1) / a.vox_per_cta), cin / 8), kWlLoad + 32, smem,
                         st>>>(a, cin, L);
@@ -1764,9 +1772,12 @@ static int bwd_w(Net& t, int l, int lvl, Src s1, Src s2, const bf16* g, cudaStre
   a.w = t.w >> lvl;
   a.err = t.err;
   t.launches += 2;
-  // lines wider than a stage holds keep the gather per tap
-  int rc = t.staged_conv && a.taps == 27 && a.w <= kWlMaxW ? wgrad_lines(kLayers[l].cin, kLayers[l].cout, a, st)
-                                                           : wgrad(kLayers[l].cin, kLayers[l].cout, a, st);
+  // Lines wider than a stage holds keep the gather per tap, and so do lines that are
+  // half padding or more: their short sums are nearly exact, and the atomics of the
+  // several times as many ranges would be most of the error (w = 4: 0.7e-7 and
+  // 2.5e-7, w = 8: 0.9e-7 and 1.8e-7).
+  const bool lines = t.staged_conv && a.taps == 27 && a.w >= kWlMinW && a.w <= kWlMaxW;
+  int rc = lines ? wgrad_lines(kLayers[l].cin, kLayers[l].cout, a, st) : wgrad(kLayers[l].cin, kLayers[l].cout, a, st);
   bias_grad(kLayers[l].cout, g, (long)a.n * a.d * a.h * a.w, t.g + t.boff[l], st);
   return rc;
 }
