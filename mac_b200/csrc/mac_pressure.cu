@@ -862,6 +862,15 @@ static int book_solve(Ctx* c, const Scalars& h) {
   return relres <= c->prm.rtol ? MAC_OK : MAC_ERR_NOT_CONVERGED;
 }
 
+// The outcome of a projection whose scalars were copied to hs_lag[2], once a later
+// read has waited for the stream. Before the later projection's own: the stats are
+// the last solve's.
+static void book_pending(Ctx* c) {
+  if (!c->lag_pending) return;
+  c->lag_status = book_solve(c, c->hs_lag[2]);
+  c->lag_pending = 0;
+}
+
 // The projection of vector field U (Divergence_Projection: divergence,
 // solve, pressure write-back, gradient correction of U). D is the speed
 // field the Dirichlet air pressures of the viscous composition read
@@ -1024,7 +1033,10 @@ int project_field(Ctx* c, double* const* U, const double* const* D, int more) {
       }
     }
     if (lagged && (rc = read_scalars(c))) return rc;
-    if (!unread) status = book_solve(c, *c->hs);
+    if (!unread) {
+      book_pending(c);
+      status = book_solve(c, *c->hs);
+    }
   } else {
     c->stats.iterations = 0;
     c->stats.relres = 0.0;
@@ -1047,8 +1059,7 @@ int project_field(Ctx* c, double* const* U, const double* const* D, int more) {
     c->lag_pending = 1;
   } else if (unread || check_div || c->lag_pending) {
     if ((rc = read_scalars(c))) return rc;
-    if (c->lag_pending) c->lag_status = book_solve(c, c->hs_lag[2]);
-    c->lag_pending = 0;
+    book_pending(c);
     if (unread) status = book_solve(c, *c->hs);
     if (check_div) {
       unsigned long long bits = c->hs->div_bits;
