@@ -152,6 +152,12 @@ void prof_end(Ctx* c, int ph) {
   c->prof->open[ph] = nullptr;
 }
 
+void prof_drop(Ctx* c, int ph) {
+  if (!c->prof || !c->prof->open[ph]) return;
+  c->prof->spare.push_back(c->prof->open[ph]);
+  c->prof->open[ph] = nullptr;
+}
+
 static void prof_resolve(Ctx* c) {
   Prof* p = c->prof;
   if (!p) return;

@@ -276,6 +276,7 @@ struct Ctx {
 
 void prof_begin(Ctx* c, int phase);
 void prof_end(Ctx* c, int phase);
+void prof_drop(Ctx* c, int phase);  // the region begun did not happen
 
 // Every kernel launch is followed by MAC_COUNT(c) so the context can report
 // how many of its kernels ran (mac_launch_count).

@@ -943,7 +943,8 @@ int project_field(Ctx* c, double* const* U, const double* const* D, int more) {
         int resident = 0;
         prof_begin(c, PH_VCYCLE);
         rc = cg_resident(c, &resident);
-        prof_end(c, PH_VCYCLE);
+        if (resident) prof_end(c, PH_VCYCLE);
+        else prof_drop(c, PH_VCYCLE);
         if (rc) return rc;
         if (resident) {
           unread = true;
