@@ -377,10 +377,13 @@ __global__ void __launch_bounds__(SPLIT ? 512 : 256) k_extrapolate(const int* __
   }
 }
 
-// Live bricks up to which the three axes get blocks of their own (us a launch, one
-// block and three): 290 bricks 17.0 and 8.9, 588 bricks 22.0 and 13.4, 2,193 bricks
-// 26.8 and 30.7 (a block of three axes shares the loads of the layers).
-constexpr int kExtrapolateSplit = 1024;
+// Live bricks up to which the three axes get blocks of their own: beyond, the blocks
+// fill the device either way, and a block of three axes shares the loads of the
+// layers and is one block to skip where nothing is written. us a pass over the
+// levels, one block a brick and three: jets of 290 bricks 54 and 41, 418 58 and 50,
+// 582 64 and 59, 797 68 and 70, 1,197 76 and 92; pools, most of whose bricks write
+// nothing, 343 27 and 34, 512 30 and 43, 1,000 40 and 66. Jets decide the line.
+constexpr int kExtrapolateSplit = 640;
 
 // Algorithms_Extrapolate on the vector field F (speed buffer 0 in pipeline A;
 // the stage speed and, through Algorithms_Accel_To_Speed, the acceleration in
