@@ -478,7 +478,9 @@ struct StagedField {
   // one bounds test for the whole stencil.
   __device__ void u8(int k, const int* key, double* out, int* bad) const {
     unsigned x = (unsigned)(key[0] - ox), y = (unsigned)(key[1] - oy), z = (unsigned)(key[2] - oz);
-    if (x + 1 < (unsigned)kStage && y + 1 < (unsigned)kStage && z + 1 < (unsigned)kStage) {
+    // (a corner one cell below the region is 2^32 - 1 here: compared without adding to it)
+    constexpr unsigned kLast = kStage - 1;
+    if (x < kLast && y < kLast && z < kLast) {
       const double* p = s + k * kStageComp + stage_slot((int)x, (int)y, (int)z);
       out[0] = p[0];
       out[1] = p[kStageZ];
