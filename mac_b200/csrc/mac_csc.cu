@@ -4,12 +4,15 @@
 // hundred thousand rows of at most seven entries, so an iteration moves a few
 // megabytes at most and its time is the latency of launches, reductions and
 // host reads: four launches, a memset and two host reads of the scalars took
-// 60 us an iteration whatever the size. Here the rows live in registers for
-// the whole solve (a row's entries, its x, r, p and its copies of the
-// neighbours' p), the blocks of one cooperative launch exchange the two dot
-// products of an iteration through tagged slots, and only z = D^-1 r passes
-// through memory (L2), as tagged words like the dots: no fence, no barrier. Measured on one B200, n = 49,542 (372 iterations):
-// 22.4 -> 1.9 ms.
+// 60 us an iteration whatever the size. Here a row stays with one thread for
+// the whole solve (its entries, its x, r, p and its copies of the neighbours' p,
+// in registers but for what the compiler spills: 128 bytes stored and 80 loaded in
+// the code of the form with 128 registers, 356 and 256 in that with 64), the blocks of
+// one cooperative launch exchange the two dot products of an iteration through
+// tagged slots, and only z = D^-1 r passes through memory (L2), as tagged words
+// like the dots: no fence, no barrier. Measured on one B200, factorise and solve,
+// launches and this kernel: n = 40,960 (127 iterations) 8.1 and 1.2 ms; with two
+// blocks an SM 79,507 (132) 9.4 and 2.2 ms, 148,877 (143) 11.4 and 3.4 ms.
 #include <cmath>
 
 #include "mac_internal.cuh"
@@ -133,6 +136,8 @@ __global__ void __launch_bounds__(kCgThreads, MINB) k_csc_cg(int n, const int* _
                                                              const double* flags, double rtol2, int max_iters,
                                                              int polls, double* out) {
   if (flags && (flags[0] != 0.0 || flags[1] != 0.0)) return;
+  __shared__ int late;  // a thread of the block gave up waiting for a neighbour's z
+  if (threadIdx.x == 0) late = 0;
   const int j = blockIdx.x * kCgThreads + threadIdx.x;
   const bool live = j < n;
   int nb[kCgRow];
@@ -180,9 +185,14 @@ __global__ void __launch_bounds__(kCgThreads, MINB) k_csc_cg(int n, const int* _
     // M = -A; the NaN of a wait that ran out ends every block's solve
     q = got ? -q : __longlong_as_double(0x7ff8000000000000ll);
     s0 = p * q;
-    ok = grid_sum<false>(s0, s1, slots, ++tag) && got;
-    // breakdown: x keeps the last finite iterate
-    if (!ok || !(s0 != 0.0 && isfinite(s0))) break;
+    ok = grid_sum<false>(s0, s1, slots, ++tag);
+    // breakdown: x keeps the last finite iterate. Whether it was a wait is asked here
+    // only: as part of every iteration's test it took 4% of one
+    if (!ok || !(s0 != 0.0 && isfinite(s0))) {
+      if (!got) late = 1;
+      __syncthreads();
+      break;
+    }
     const double alpha = rz / s0;
     xs += alpha * p;
     r -= alpha * q;
@@ -206,7 +216,7 @@ __global__ void __launch_bounds__(kCgThreads, MINB) k_csc_cg(int n, const int* _
     out[1] = rr;
     out[2] = bb;
   }
-  if (!ok) out[3] = 1.0;
+  if (threadIdx.x == 0 && (!ok || late)) out[3] = 1.0;
 }
 
 // Enqueues the whole solve of A x = b (A symmetric with a negative diagonal,
