@@ -839,6 +839,7 @@ __global__ void __launch_bounds__(kWlLoad + 32) k_wgrad_lines(WgradArgs a, int c
   const int l1 = len > 0 ? min(V / a.w, a0 + len + a.h) : 0;
   // the first line from `line` on that the range meets
   auto meets = [&](int line) -> int {
+    if (len >= a.h) return line;  // no gaps
     const int r = (line - (a0 - a.h)) % a.h;
     return r < len ? line : min(l1, line + a.h - r);
   };
