@@ -1400,21 +1400,21 @@ static void conv_tile_t(const ConvArgs& a, cudaStream_t st) {
   k_conv_tile<KC, NC><<<(unsigned)tiles, 128, smem, st>>>(a);
 }
 
-// Planes a CTA walks: as long a run as still gives the device a few CTAs an SM
-// (a run stages the weights and two extra planes), in runs of equal length of at
-// least four planes, or of fewer where the grid would otherwise have less than 1.5
-// CTAs an SM (a run's planes follow one another, so four of them are six times a
-// plane's latency). us a forward pass: a CTA a plane with its box staged at once,
-// always four planes, this rule: 1 x 8^3 174, 225, 175; 1 x 128 x 8 x 8 176, 234, 179;
-// 16 x 16^3 207, 234, 192; 1 x 36^3 218, 234, 195. Lines at 1, 2, 3 and 4 CTAs an SM:
-// 16 x 16^3 200, 189, 189, 190; 16 x 20^3 252, 274, 274, 283; 1 x 100 x 84 x 60 404,
-// 428, 427, 469.
+// Planes a CTA walks: as long a run as still gives the device `want` CTAs, what it
+// holds at a time (a run stages the weights and two extra planes), in runs of equal
+// length of at least four planes, or of fewer where the grid would otherwise have less
+// than 1.5 CTAs an SM (a run's planes follow one another, so four of them are six times
+// a plane's latency), never more than fit at a time.
+// us a forward pass: a CTA a plane with its box staged at once, always four planes, this
+// rule: 1 x 8^3 167, 217, 169; 1 x 128 x 8 x 8 175, 231, 177; 16 x 16^3 207, 232, 191;
+// 1 x 36^3 216, 233, 193; 16 x 20^3 345, 250, 235 (250 where the CTAs may exceed what
+// fits); 16 x 64^3 3,675, 1,473, 1,474 (1,488).
 static int march_run(const long tiles, int d, int want) {
   long runs = (want + tiles - 1) / tiles;
   if (runs < 1) runs = 1;
   if (runs > (d + 3) / 4) runs = (d + 3) / 4;
-  constexpr long kFew = 148 * 3 / 2;
-  if (tiles * runs < kFew) runs = std::min<long>(d, (kFew + tiles - 1) / tiles);
+  const long few = std::min<long>(148 * 3 / 2, want);
+  if (tiles * runs < few) runs = std::max(runs, std::min<long>(d, few / tiles));
   return (int)((d + runs - 1) / runs);
 }
 
