@@ -1480,11 +1480,14 @@ static void wgrad_lines_t(int cin, WgradArgs a, cudaStream_t st) {
   const int w16 = (a.w + 15) / 16 * 16;
   a.vox_per_cta = wgrad_range(cin, 27, V);
   // Padded lines take w16 / w times the MMAs for the same voxels, each of which
-  // truncates the sum it adds to: whole lines, at most half as many MMAs a sum as
-  // k_wgrad's range has. Error against 64 bits in multiples of k_wgrad's, with its
-  // ranges and with these: lines of 40 (16 columns) 1.0 and 0.35, of 20 (32 columns)
-  // 1.1 and 0.24, of 10 (64 columns) 1.4 and 0.4. The times are the same.
-  if (a.w % 16) a.vox_per_cta = std::max(1, a.vox_per_cta / (2 * w16)) * a.w;
+  // truncates the sum it adds to: whole lines, at most three quarters of the MMAs that
+  // a sum of k_wgrad's range has. Error against 64 bits in multiples of k_wgrad's, with
+  // its ranges and with these: lines of 40 (16 columns) 1.0 and 0.53, of 20 (32
+  // columns) 1.1 and 0.46, of 10 (64 columns) 1.4 and 0.63. ms a loss and gradient with
+  // its ranges, with these and with half the MMAs: 16 x 64 x 64 x 40 7.24, 6.72, 7.18,
+  // 1 x 100 x 84 x 60 2.55, 2.61, 2.86 (more ranges than fit at a time), 8 x 40^3 2.52,
+  // 2.53, 2.77.
+  if (a.w % 16) a.vox_per_cta = std::max(1, (int)(3L * a.vox_per_cta / (4 * w16))) * a.w;
   const int L = wl_vox<COUT>() / w16, smem = 2 * wl_stage<COUT>(a.w, L);
   cudaFuncSetAttribute(k_wgrad_lines<COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   k_wgrad_lines<COUT><<<dim3((unsigned)((V + a.vox_per_cta - 1) / a.vox_per_cta), cin / 8), kWlLoad + 32, smem,

@@ -8,7 +8,7 @@ unchanged in its bits (times 8 and 64). The gradient of a tap's weight is then a
 sum of BF16 numbers that FP64 adds exactly, and what a device sum is off is its
 own rounding. The exponents spread over 14 bits, so a sum needs more than FP32 has.
 
-The staged sums take at most half as many additions as the per-tap kernels'
+The staged sums take at most three quarters of the additions of the per-tap kernels'
 (set_conv(False)), so their error is no larger but for the FP32 atomics that join
 the ranges: up to 300, each rounding to nearest, 2^-24 sqrt(300) together.
 """
