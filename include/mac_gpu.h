@@ -252,7 +252,9 @@ int mac_get_profile(void* ctx, double* ms, int64_t* count, int nphase);
  * device; any other matrix (the general LU of Umfpack takes any non-singular one) by
  * FP64 Jacobi-preconditioned BiCGStab on a row-major copy. Both stop at
  * ||b - A x|| <= rtol ||b|| (mac_params.rtol) or return MAC_ERR_NOT_CONVERGED after
- * max_iters or on a breakdown, with x the last finite iterate. ---- */
+ * max_iters or on a breakdown, with x the last finite iterate. mac_csc_clean drops
+ * the matrix; up to 64 MB of its device memory stays with the context for the next
+ * one (mac_ctx_destroy gives it back), more is freed at once. ---- */
 int mac_csc_factorize(void* ctx, int n, const int* offset, const int* indice, const double* value);
 int mac_csc_solve(void* ctx, int n, const double* b, double* x);
 int mac_csc_clean(void* ctx);
@@ -271,7 +273,10 @@ int mac_unet_nparams(void* net, int64_t* n);
 int mac_unet_init(void* net, uint64_t seed);
 int mac_unet_get_params(void* net, float* params, float* tscale);
 int mac_unet_set_params(void* net, const float* params, float tscale);
-/* out = net(r / rms(r), mask) * rms(r) * tscale on fluid cells, 0 elsewhere (host arrays). */
+/* out = net(r / rms(r), mask) * rms(r) * tscale on fluid cells, 0 elsewhere (host arrays).
+ * This call and mac_unet_loss_grad move pageable arrays of 2 MB or more in all through
+ * 4 MB of pinned memory of the network (made on first use, freed with it), by
+ * the calling thread and three more that end with the copy. */
 int mac_unet_forward(void* net, int n, int d, int h, int w, const float* r, const int8_t* mask, float* out);
 /* loss = mean over fluid cells of (net(r / rms(r), mask) - e / (rms(r) tscale))^2 and its
  * gradient with respect to every parameter (host arrays). */
@@ -380,8 +385,9 @@ int mac_set_smoother(void* ctx, double w1, double w2, double w_single, double co
  *   Its reduction slots must be zero before each reduction, and the call clears
  *   them itself, so the caller prepares nothing.
  * - Runs on `stream` (a cudaStream_t, 0 for the legacy stream) on the current
- *   device and returns after the solve has finished (it reads the CG scalars
- *   on the host every iteration).
+ *   device and returns after the solve has finished. Matrices of at most seven
+ *   entries a column are checked and solved with one host read in all; for
+ *   longer columns the CG scalars are read on the host every iteration.
  * - The first call on a device looks up the array's address with
  *   cudaGetSymbolAddress; the driver then places the array (2.5 MiB) in device
  *   memory, so that first call needs that much free. A call with n = 0 does

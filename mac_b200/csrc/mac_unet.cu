@@ -569,6 +569,8 @@ __global__ void __launch_bounds__(128) k_wgrad(WgradArgs a) {
 // B200 (first a box per output plane or a gather per tap in MODE 1, then a march
 // with one dz an MMA, now), us: forward at 128^3, 16 -> 16 channels 166, 108, 83,
 // 32 -> 16 569, 320, 158; input gradient of 16 x 64^3, 16 -> 16 812, 231, 122.
+// What bounds it now are the planes' loads and the barrier between planes: at
+// 4 x 64^3 the tensor pipe is active 19-21% of the time, issue slots 29-43%.
 constexpr int kPlX = 10, kPlY = 18, kPlVox = kPlX * kPlY;
 
 // Shared memory, accumulators in the ring and CTAs an SM: eight accumulators
@@ -787,6 +789,8 @@ __global__ void __launch_bounds__(128, March<KC, NC>::occ) k_conv_march(ConvArgs
 // issues the MMAs of a step while sixteen load the next. Measured on one B200
 // (before: k_wgrad), 16 x 64^3 samples: the four layers of 16 columns 11.2 -> 2.5
 // ms, of 32 columns (half resolution) 4.2 -> 1.1 ms.
+// What bounds it now is the staging (4 x 64^3, 16 columns: issue slots 46-50% used,
+// tensor pipe active 11-12%).
 constexpr int kWlLoad = 512;  // loading threads; a further warp issues the MMAs
 constexpr int kWlIn = 2;      // chunks of input lines a thread carries
 constexpr int kWlVox = 256;   // voxels of a step, padding included
@@ -1559,7 +1563,9 @@ struct Net {
 // that copy a chunk in or out while the link moves others. Registered or device
 // memory, small arrays and a failed staging allocation take the plain copy.
 // Measured on one B200 (16 cores): forward at 128^3 (10.5 MB in, 8.4 MB out) 3.15
-// -> 2.25 ms, loss and gradient of 16 x 64^3 (38 MB in) 11.0 -> 9.3 ms.
+// -> 2.25 ms, loss and gradient of 16 x 64^3 (38 MB in) 11.0 -> 9.3 ms. Making the
+// buffer takes 2.5 to 5 ms, once a network (its first forward at 128^3 18.0 -> 20.8 ms;
+// with chunks of 256 KB 19.3, but the gradient 9.6).
 constexpr int kCopyLanes = 4;
 constexpr size_t kCopyChunk = 512 * 1024, kCopyMin = 2 * 1024 * 1024;
 struct HostCopy {
