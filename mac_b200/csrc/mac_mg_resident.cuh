@@ -4,7 +4,7 @@
 // A CG iteration of the launch-by-launch form is some twenty dependent kernels,
 // each a few microseconds of launch, ramp-up and one or two rounds of load
 // latency, so an iteration took 65-80 us however small the system was. Here one
-// block an SM (or one cluster of up to 16 blocks, up to 64 bricks) runs
+// block an SM (or one cluster of up to 16 blocks, for the smallest systems) runs
 // every phase of every iteration; phases are separated by a grid-wide exchange
 // that also carries the dot products, static data of the next phase is loaded
 // while a block waits, the coarse levels stay in block 0's shared memory for the
@@ -942,15 +942,8 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const __grid_con
 }
 
 // Systems of at most this many domain bricks go to one cluster of at most
-// kResCluster blocks: a brick a group. A second round of bricks costs a phase more
-// than the cluster's exchanges save (us an iteration, FP64, one cluster and the grid:
-// 48 bricks 26 and 30, 64 29 and 30, 72 39 and 33, 108 43 and 34; FP32 levels 24 and
-// 28, 25 and 28, 34 and 31, 37 and 31).
-constexpr int kResClusterBricks = kResCluster * kResGroups;
-// Level 2 joins block 0's levels up to this many cells (ms a projection, with it and
-// with level 2 spread over the blocks: 18 bricks of a 3 x 3 x 3 box 0.43 and 0.50, 512
-// of 8 x 8 x 8 (4,096 cells) 0.93 and 0.94; past the line, 490 of 9 x 9 x 9, 0.94 and
-// 0.89).
+// kResCluster blocks, and level 2 joins block 0's levels up to this many cells.
+constexpr int kResClusterBricks = 128;
 constexpr int kResBlk2 = 4096;
 
 template <class T>
