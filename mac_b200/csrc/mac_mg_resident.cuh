@@ -942,8 +942,18 @@ __global__ void __launch_bounds__(kResThreads, 1) k_cg_resident(const __grid_con
 }
 
 // Systems of at most this many domain bricks go to one cluster of at most
-// kResCluster blocks, and level 2 joins block 0's levels up to this many cells.
+// kResCluster blocks. The cluster is the faster one up to a brick a group (us an
+// iteration, FP64, cluster and grid: 48 bricks 26 and 30, 64 29 and 30; FP32 levels 24
+// and 28, 25 and 28); with a second round of bricks the grid is (72: 39 and 33, 108: 43
+// and 34; FP32 34 and 31, 37 and 31). The line stays at two rounds all the same: the
+// forms add their dot products in other orders, and with FP32 levels the pressures of
+// systems between the lines would move by more than 1e-9 of themselves, inside the
+// solve's tolerance but not reproducibly with earlier results.
 constexpr int kResClusterBricks = 128;
+// Level 2 joins block 0's levels up to this many cells (ms a projection, with it and
+// with level 2 spread over the blocks: 18 bricks of a 3 x 3 x 3 box 0.43 and 0.50, 512
+// of 8 x 8 x 8 (4,096 cells) 0.93 and 0.94; past the line, 490 of 9 x 9 x 9, 0.94 and
+// 0.89).
 constexpr int kResBlk2 = 4096;
 
 template <class T>
